@@ -271,7 +271,7 @@ int alloc_grid(wx_ctx *ctx, const std::vector<int4> &o5, uint64_t n5, uint64_t n
         return fail(ctx, WX_ERR_OOM, "host allocation failed");
     }
     auto align = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    const size_t b_o5 = align(root.size() * 16), b5 = align(n5 * 32768ull * 4),
+    const size_t b_top = wxk::kTopWords * sizeof(uint32_t), b_o5 = align(root.size() * 16) + b_top, b5 = align(n5 * 32768ull * 4),
                  b4 = align(n4 * 4096ull * 4), b3 = align(n3 * 512ull), bo = align(n_ovf * 8);
     gr->bytes = b_o5 + b5 + b4 + b3 + bo;
     gr->device = ctx->device;
@@ -316,9 +316,11 @@ void free_grid(wx_grid *gr) {
 }
 
 // Pack the per-voxel u32 leaf distances into bytes plus the overflow table,
-// allocate one device block for all pools and upload them.
+// allocate one device block for all pools and upload them. far_tiles: some N5 or N4 distance is
+// 2^24 or more (a hand-made view; compute_sdf's stay below 2000, the side of the largest cube of
+// nodes that a grid can hold).
 int upload_pools(wx_ctx *ctx, const std::vector<int4> &o5, const uint32_t *s5, const uint32_t *s4, const uint32_t *s3,
-                 uint64_t n5, uint64_t n4, uint64_t n3, wx_grid **out) {
+                 uint64_t n5, uint64_t n4, uint64_t n3, bool far_tiles, wx_grid **out) {
     int rc = check_pool_limits(ctx, n5, n4, n3);
     if (rc != WX_OK) return rc;
     std::vector<uint8_t> leaf;
@@ -352,6 +354,9 @@ int upload_pools(wx_ctx *ctx, const std::vector<int4> &o5, const uint32_t *s5, c
     if (e == cudaSuccess && n3) e = cudaMemcpy((void *)gr->g.leaf, leaf.data(), leaf.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !ovf.empty())
         e = cudaMemcpy((void *)gr->g.ovf, ovf.data(), ovf.size() * 8, cudaMemcpyHostToDevice);
+    if (far_tiles) gr->g.inside |= 2u;
+    if (e == cudaSuccess) e = wxk::build_top_table(gr->g, nullptr);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
         free_grid(gr);
         return cuda_fail(ctx, e, "cudaMemcpy(node pools)");
@@ -658,7 +663,7 @@ int wx_grid_build(wx_ctx *ctx, wx_topology *t, wx_grid **out) {
         }
         if (too_far) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build: tile distance >= 2^31");
         wx_grid *gr = nullptr;
-        rc = upload_pools(ctx, o5, s5.data(), s4.data(), t->slot3.data(), n5, n4, n3, &gr);
+        rc = upload_pools(ctx, o5, s5.data(), s4.data(), t->slot3.data(), n5, n4, n3, false, &gr);
         if (rc != WX_OK) return rc;
         gr->info.active_voxels = wx_topology_active_voxels(t);
         *out = gr;
@@ -783,6 +788,7 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
         if (e == cudaSuccess)
             e = wxk::sdf_pack_leaves(d3.as<uint32_t>(), n3 * kN3Slots, const_cast<uint8_t *>(gr->g.leaf),
                                      const_cast<uint2 *>(gr->g.ovf), (uint32_t)n_ovf, flags + 3, st);
+        if (e == cudaSuccess) e = wxk::build_top_table(gr->g, st);
         if (e == cudaSuccess) e = cudaMemcpy(h, flags, sizeof h, cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) {
             free_grid(gr);
@@ -862,6 +868,7 @@ int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *v, wx_grid **out) {
             return fail(ctx, WX_ERR_OOM, "wx_grid_upload: host allocation failed");
         }
         std::atomic<int> bad{0};
+        std::atomic<bool> far{false};
         for (uint64_t i = 0; i < n5; i++) {
             const int32_t *o = v->origins + i * v->origin_stride;
             o5[i] = make_int4(o[0], o[1], o[2], 0);
@@ -877,7 +884,7 @@ int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *v, wx_grid **out) {
                     uint32_t word;
                     if (val) word = 0;
                     else if (kid) { word = wx::kChildFlag | tx; if (tx >= n4) bad = 1; }
-                    else { word = tx; if (tx >= wx::kChildFlag) bad = 2; }
+                    else { word = tx; if (tx >= wx::kChildFlag) bad = 2; else if (tx >= (1u << 24)) far = true; }
                     s5[i * wx::kN5Slots + s] = word;
                 }
         });
@@ -892,7 +899,7 @@ int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *v, wx_grid **out) {
                     uint32_t word;
                     if (val) word = 0;
                     else if (kid) { word = wx::kChildFlag | tx; if (tx >= n3) bad = 1; }
-                    else { word = tx; if (tx >= wx::kChildFlag) bad = 2; }
+                    else { word = tx; if (tx >= wx::kChildFlag) bad = 2; else if (tx >= (1u << 24)) far = true; }
                     s4[j * wx::kN4Slots + s] = word;
                 }
         });
@@ -908,7 +915,7 @@ int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *v, wx_grid **out) {
         if (bad == 1) return fail(ctx, WX_ERR_INVALID, "wx_grid_upload: child index in atlas out of range");
         if (bad == 2) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_upload: internal tile distance >= 2^31");
         wx_grid *gr = nullptr;
-        int rc = upload_pools(ctx, o5, s5.data(), s4.data(), s3.data(), n5, n4, n3, &gr);
+        int rc = upload_pools(ctx, o5, s5.data(), s4.data(), s3.data(), n5, n4, n3, far, &gr);
         if (rc != WX_OK) return rc;
         uint64_t act = 0;
         for (uint64_t w = 0; w < n3 * 16; w++) act += (uint64_t)__builtin_popcount(v->vals3[w]);

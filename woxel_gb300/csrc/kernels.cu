@@ -44,7 +44,7 @@ __device__ __forceinline__ bool tile_pixel(const Job &J, uint32_t tl, uint32_t l
     return gx < (J.width & ~7u) && gy < (J.height & ~3u);
 }
 
-template <bool kAll, bool kFmaStep01 = true>
+template <bool kAll, bool kCompact = false>
 __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t lane, bool wait_prev) {
     uint32_t gx, gy;
     // The warp's lanes leave each march at different iterations. Without the
@@ -56,7 +56,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
     const wx_state_uniform &s = J.s;
     const F3 dir = primary_dir(s, gx, gy);
     const F3 eye = f3(s.eye[0], s.eye[1], s.eye[2]);
-    const March hit = hdda<kFmaStep01>(J.g, eye, dir);
+    const March hit = hdda(J.g, eye, dir);
     __syncwarp(act);
     F3 c;
     uint32_t shadow = 0, reserved = 0;
@@ -81,7 +81,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
             F3 shadowed, src;
             c = primary_colour(s, hit, dir, &need, &shadowed, &src);  // states 1, 2: mode 3's colours
         }
-    } else if (!kFmaStep01) {  // modes 0-3 in the persistent kernels
+    } else if (kCompact) {  // modes 0-3 in the persistent kernels
         // Everything the stores need is reduced to a few words before the shadow
         // march (the packed colour, t, the info word), so that the direction and
         // both candidate colours are not live across it: the persistent kernels
@@ -97,7 +97,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
         const uint32_t node = hit.node;
         __syncwarp(act);  // shadow rays of the warp start together
         if (need) {
-            const March sh = hdda<kFmaStep01>(J.g, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
+            const March sh = hdda(J.g, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
             shadow = 1u | (sh.state << 1) | (sh.i << 8);
             if (sh.state == 0u) cpk = pack_rgba(ambient_colour());  // shadowed is I_a
         }
@@ -114,7 +114,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
         c = primary_colour(s, hit, dir, &need, &shadowed, &src);
         __syncwarp(act);  // shadow rays of the warp start together
         if (need) {
-            const March sh = hdda<kFmaStep01>(J.g, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
+            const March sh = hdda(J.g, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
             shadow = 1u | (sh.state << 1) | (sh.i << 8);
             if (sh.state == 0u) c = shadowed;
         }
@@ -133,17 +133,15 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
                   hit.state | (hit.np << 2) | (hit.mask << 4) | (hit.i << 8), shadow, reserved);
 }
 
-// Blocks of at most 256 threads. The persistent kernels: at least 5 resident,
-// 48 registers a thread and 40 resident warps per SM. k_pixel: at least 6, 40
-// registers and 48 warps (modes 0-3; the kernel of every mode keeps 48 registers,
-// which its glossy and zero-crossing code needs). Measured on GB300 (16 frames of 2000 spheres at
-// 1080p): k_pixel 3.34 Grays/s at 40 registers against 3.17 at 48 and 3.30 at 32
-// (its finished blocks retire while the previous frame ends, so more resident warps
-// pay); the persistent kernels are slower at 40 registers (the mixed batch 4.38
-// against 4.80 Grays/s at 48; spills in the march loop) and beat 64 (32 warps) by 2%
-// and 80 (24 warps) by 17% at 48.
+// Blocks of at most 256 threads. k_pixel in modes 0-3: 8 resident, 32 registers a thread, all 64
+// warp slots of an SM. Its march waits on dependent loads and leaves a third of its lanes idle, so
+// resident warps pay more than the five reloads an iteration that 32 registers cost: 8 frames of
+// 2000 spheres at 1080p take 3.27 ms at 32 registers, 3.47 at 40 and 3.67 at 47 (2 noise frames at
+// 4K: 2.20, 2.23 and 2.29 ms). Its kernel of every mode keeps 48 registers for the glossy and
+// zero-crossing code. The persistent kernels hold the job's pointers in registers and stay at 48
+// (5 blocks, 40 warps): 48 mixed frames take 13.0 ms, 14.2 at 40 registers and 13.4 at 55.
 #define WX_RAY_BOUNDS __launch_bounds__(256, 5)
-#define WX_PIXEL_BOUNDS __launch_bounds__(256, kAll ? 5 : 6)
+#define WX_PIXEL_BOUNDS __launch_bounds__(256, kAll ? 5 : 8)
 
 // One warp per tile of one frame, tiles in block order (rows in the job's order).
 // Frames on one stream overlap in time: the next k_pixel starts once every block
@@ -412,11 +410,22 @@ __global__ void WX_RAY_BOUNDS k_persistent(const Job *__restrict__ jobs, uint32_
                     continue;
                 }
             }
-            render_pixel<kAll, false>(J, t - J.tile_begin + J.tile_off, lane, true);
+            render_pixel<kAll, true>(J, t - J.tile_begin + J.tile_off, lane, true);
         } else {
-            render_pixel<kAll, false>(job0, t, lane, true);
+            render_pixel<kAll, true>(job0, t, lane, true);
         }
     }
+}
+
+// The dense table of the box's N5 slot words (wxk::kTopWords). An absent N5 reads as tiles of
+// distance 32: 32 * 128 voxels is the 4096 that the march uses where no N5 is found.
+__global__ void k_top_table(DevGrid g) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= wxk::kTopWords) return;
+    const uint32_t x = i >> 12, y = (i >> 6) & 63u, z = i & 63u;
+    const uint32_t n = root_find(g, (int)(x << 7) - 4096, (int)(y << 7) - 4096, (int)(z << 7) - 4096);
+    const_cast<uint32_t *>(g.slot5)[(int)i - (int)wxk::kTopWords] =
+        n == kNoNode ? 32u : g.slot5[(n << 15) | ((x & 31u) << 10) | ((y & 31u) << 5) | (z & 31u)];
 }
 
 __global__ void k_check_div(uint32_t max_m, unsigned long long *out) {
@@ -466,6 +475,11 @@ cudaError_t init_device_tables() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_wave<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, wave_max);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_wave<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, wave_max);
     return e;
+}
+
+cudaError_t build_top_table(const DevGrid &g, cudaStream_t st) {
+    k_top_table<<<kTopWords / 256, 256, 0, st>>>(g);
+    return cudaGetLastError();
 }
 
 int max_blocks_per_sm(int kernel, bool batched, int warps_per_block) {

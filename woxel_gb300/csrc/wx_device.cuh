@@ -195,7 +195,7 @@ __device__ __forceinline__ uint32_t root_find(const DevGrid &g, int x, int y, in
 // r.i is the iteration count the shader reports. kCareful selects the
 // NaN-aware min/argmin and the literal nudge (see ray_needs_careful_step);
 // both variants give identical results on the rays the fast one is used for.
-template <bool kCareful, bool kFmaStep01 = true>
+template <bool kCareful>
 __device__ __forceinline__ uint32_t ray_step(const DevGrid &g, Ray &r) {
     if (r.i >= kMaxSteps) return 2u;
     // vec3<i32>(floor(p)): one saturating round-down conversion (NaN -> 0).
@@ -271,10 +271,7 @@ __device__ __forceinline__ uint32_t ray_step(const DevGrid &g, Ray &r) {
     // step01 = max(0, sign11(dir)): 0 where dir < 0, else 1. The fast step only
     // takes rays whose direction components are nonzero numbers, for which
     // copysign(0.5, d) + 0.5 gives the same 0 or 1 (on the FMA pipe).
-    // kFmaStep01 = false keeps the compare-and-select form in the fast step too:
-    // the persistent kernels spill more with the copysign form and run slower
-    // with it (4.45 -> 4.32 Grays/s on the mixed batch), while k_pixel gains.
-    constexpr bool kSel = kCareful || !kFmaStep01;
+    constexpr bool kSel = kCareful;
     const float ax = kSel ? (r.dx < 0.0f ? 0.0f : 1.0f) : __fadd_rn(copysignf(0.5f, r.dx), 0.5f);
     const float ay = kSel ? (r.dy < 0.0f ? 0.0f : 1.0f) : __fadd_rn(copysignf(0.5f, r.dy), 0.5f);
     const float az = kSel ? (r.dz < 0.0f ? 0.0f : 1.0f) : __fadd_rn(copysignf(0.5f, r.dz), 0.5f);
@@ -366,20 +363,141 @@ __device__ __forceinline__ March march_result(const Ray &r, uint32_t st) {
     return m;
 }
 
-// hdda_ray (raycast.comp.wgsl:84-126) run to completion.
-template <bool kFmaStep01 = true>
-__device__ __forceinline__ March hdda(const DevGrid &g, F3 src, F3 dir) {
+// hdda_ray by ray_step, from position p after i iterations whose last mask is mask: every
+// grid and every ray. The lookup of a step does not depend on the cached chain, so the march
+// may start at any iteration.
+__device__ __forceinline__
+March hdda_general(const DevGrid &g, F3 p, F3 dir, uint32_t i, uint32_t mask) {
     Ray r;
-    ray_init(r, src, dir);
+    ray_init(r, p, dir);
+    r.i = i;
+    r.mx = mask & 1u;
+    r.my = mask & 2u;
+    r.mz = mask & 4u;
     uint32_t st;
-    if (ray_needs_careful_step(src, dir)) {
-        while ((st = ray_step<true, kFmaStep01>(g, r)) == 0xFFu) {
-        }
-    } else {
-        while ((st = ray_step<false, kFmaStep01>(g, r)) == 0xFFu) {
-        }
+    while ((st = ray_step<true>(g, r)) == 0xFFu) {
     }
     return march_result(r, st);
+}
+
+// floor by the adder: for |p| < 2^21, RD(p + kFloorMagic) is the float kFloorMagic + floor(p),
+// whose bits are 0x4B400000 + (floor(p) + 4096): the low 22 bits are the voxel coordinate moved
+// into the [0, 8192) box, and subtracting kFloorMagic gives floor(p) exactly. Any other p (larger,
+// infinite, NaN) leaves bits outside 0x4B400000 + [0, 8192).
+constexpr float kFloorMagic = 12582912.0f + 4096.0f;
+constexpr uint32_t kBoxBits = 0x4B400000u, kBoxSide = 8192u;
+
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+// hdda_ray (raycast.comp.wgsl:84-126) run to completion.
+//
+// The loop below performs the shader's iterations on the rays that need no care
+// (ray_needs_careful_step), with the same results bit for bit; what it does not cover leaves it and
+// is finished by hdda_general from the state reached: a position outside the box [-4096, 4096)^3
+// that does not end the ray, and a coordinate in (-2^-64, 0).
+//  * Lookup. Inside the box the N5 slot words of all octants form one dense table (64^3 words before
+//    slot5; 32 fills a missing N5: a tile of 32 * 128 = 4096 voxels, the size an absent N5 has), so a
+//    lookup is at most three loads and needs no root search. scl is the size scale of the level that
+//    resolved the previous lookup (1, 8, 128; 4096 outside the box): or-ed into the XOR of the
+//    voxel coordinates it also says which cached node may be reused, since a node of side S holds the
+//    new voxel exactly if that XOR is below S.
+//  * floor(p / size) is the floor of the correctly rounded quotient in the shader, and that equals
+//    floor(p / size) itself: for K = k * size, the float next to K on either side is a relative
+//    2^-24 or more away, more than half an ulp of k, so no quotient rounds onto or across k (only a
+//    quotient that underflows could: -2^-64 < p < 0 is left to hdda_general). size is an integer,
+//    so it is also floor((floor(p) + 0.5) / size), at least 0.5 / size away from any
+//    integer: with |floor(p) + 0.5| < 4097 an approximate reciprocal (relative error 2^-22) is
+//    exact enough by a factor of 2^9.
+//  * The products and sums of tMax are exact or rounded once, as in ray_step.
+// Bound by instruction issue (81-88% of the slots) at 20 to 29 of 32 lanes, then by the three
+// dependent loads. Against ray_step<false> in the same kernels: about 106 instead of 132 warp
+// instructions an iteration, no root search, and no table load between the lookup and the
+// quotients; 8 frames of 2000 spheres at 1080p 4.64 -> 3.27 ms, 2 noise frames at 4K 2.97 -> 2.20 ms,
+// 48 mixed frames in one batch 18.1 -> 13.0 ms, one 160x120 frame 33 -> 27 us.
+// Tried and slower there: keeping the mask as three bools (3.41 ms for the 8 frames), any form that
+// lets the compiler turn the level blocks into predicated straight-line code (a box test without a
+// branch 3.57 ms, the leaf overflow handled outside the loop 3.77 ms), floor by a second addition
+// instead of FRND (+1%), step01 by compare and select (3.47), a second loop for warps whose
+// directions have one sign pattern (no change).
+__device__ __forceinline__ March hdda(const DevGrid &g, F3 src, F3 dir) {
+    if (ray_needs_careful_step(src, dir) || (g.inside & 2u)) return hdda_general(g, src, dir, 0u, 0u);
+    float px = src.x, py = src.y, pz = src.z;
+    const float ix = __frcp_rn(dir.x), iy = __frcp_rn(dir.y), iz = __frcp_rn(dir.z);
+    uint32_t lx = 0, ly = 0, lz = 0, scl = 4096u, i4 = 0, i3 = 0, i = 0, w;
+    float t = 0.0f, tx = 1.0f, ty = 1.0f, tz = 1.0f;  // the last step's mask is tx == t, ty == t, tz == t
+    do {
+        const float rx = __fadd_rd(px, kFloorMagic), ry = __fadd_rd(py, kFloorMagic), rz = __fadd_rd(pz, kFloorMagic);
+        const uint32_t x = __float_as_uint(rx), y = __float_as_uint(ry), z = __float_as_uint(rz);
+        const uint32_t d = (x ^ lx) | (y ^ ly) | (z ^ lz) | scl;
+        lx = x; ly = y; lz = z;
+        w = kChild;
+        if (d >= 128u) {  // get_vdb_leaf_from_nothing / from_node5 (:398-444)
+            w = 0u;
+            scl = 4096u;
+            if (((x | y | z) ^ kBoxBits) < kBoxSide) {
+                const uint32_t idx = ((x & 0x1F80u) << 5) | ((y >> 1) & 0xFC0u) | ((z >> 7) & 0x3Fu);
+                w = __ldg(g.slot5 - wxk::kTopWords + idx);
+                i4 = w << 12;
+                scl = 128u;
+            }
+        }
+        if (d >= 8u && (int)w < 0) {  // get_vdb_leaf_from_node4 (:446-475)
+            const uint32_t idx = i4 + (((x & 0x78u) << 5) | ((y & 0x78u) << 1) | ((z >> 3) & 15u));
+            w = 0u;
+            if (wx_in_range(i4 >> 12, g.n4)) w = __ldg(g.slot4 + idx);
+            i3 = w << 9;
+            scl = 8u;
+        }
+        if ((int)w < 0) {  // get_vdb_leaf_from_node3 (:477-494)
+            const uint32_t key = i3 + (((x & 7u) << 6) | ((y & 7u) << 3) | (z & 7u));
+            w = 0u;
+            if (wx_in_range(i3 >> 9, g.n3)) w = __ldg(g.leaf + key);
+            if (w == 255u) w = leaf_overflow(g, key);
+            scl = 1u;
+        }
+        const uint32_t s = w * scl;  // grids with tile distances of 2^24 or more are marched by hdda_general
+        if (s == 0u || min(min(__float_as_int(px), __float_as_int(py)), __float_as_int(pz)) < (int)0x9F800000) break;
+        const float size = __uint2float_rn(s), rc = rcp_approx(size), hf = 0.5f * rc;
+        const float ax = __fadd_rn(copysignf(0.5f, dir.x), 0.5f);
+        const float ay = __fadd_rn(copysignf(0.5f, dir.y), 0.5f);
+        const float az = __fadd_rn(copysignf(0.5f, dir.z), 0.5f);
+        const float fx = floorf(__fmaf_rn(rx - kFloorMagic, rc, hf));
+        const float fy = floorf(__fmaf_rn(ry - kFloorMagic, rc, hf));
+        const float fz = floorf(__fmaf_rn(rz - kFloorMagic, rc, hf));
+        tx = ix * __fmaf_rn(size, ax, -__fmaf_rn(-size, fx, px));
+        ty = iy * __fmaf_rn(size, ay, -__fmaf_rn(-size, fy, py));
+        tz = iz * __fmaf_rn(size, az, -__fmaf_rn(-size, fz, pz));
+        t = fminf(fminf(tx, ty), tz);
+        const bool mx = tx == t, my = ty == t, mz = tz == t;
+        px = px + t * dir.x;
+        py = py + t * dir.y;
+        pz = pz + t * dir.z;
+        const float kNudge = 0.5f * 8e-4f;
+        const float nx = copysignf(kNudge, dir.x), ny = copysignf(kNudge, dir.y), nz = copysignf(kNudge, dir.z);
+        px = mx ? px + nx : px;
+        py = my ? py + ny : py;
+        pz = mz ? pz + nz : pz;
+    } while (++i < kMaxSteps);
+    const bool mx = tx == t, my = ty == t, mz = tz == t;
+    March m;
+    m.mask = (uint32_t)mx | ((uint32_t)my << 1) | ((uint32_t)mz << 2);
+    m.state = i == kMaxSteps ? 2u : w != 0u ? 3u : scl != 4096u ? 0u : 1u;
+    if (m.state == 1u && !(g.inside == 1u && 4096.0f < fmaxf(fmaxf(fabsf(px), fabsf(py)), fabsf(pz)))) m.state = 3u;
+    if (m.state == 3u) return hdda_general(g, f3(px, py, pz), dir, i, m.mask);
+    m.p = f3(px, py, pz);
+    m.i = i;
+    m.np = scl == 1u ? 3u : scl == 8u ? 2u : 0u;
+    m.node = scl == 1u ? i3 >> 9 : scl == 8u ? i4 >> 12 : kNoNode;
+    if (scl == 128u) {  // an N5's slot, or a missing N5
+        m.node = root_find(g, (int)(lx & (kBoxSide - 1u)) - 4096, (int)(ly & (kBoxSide - 1u)) - 4096,
+                           (int)(lz & (kBoxSide - 1u)) - 4096);
+        m.np = m.node != kNoNode ? 1u : 0u;
+    }
+    return m;
 }
 
 __device__ __forceinline__ F3 maskf(uint32_t m) {

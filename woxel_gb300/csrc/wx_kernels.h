@@ -19,9 +19,14 @@ struct DevGrid {
     const float *values;     // level-set value per leaf voxel (zero-crossing mode), or null
     uint32_t n5, n_ovf;
     float band;              // value of voxels outside leaves (+band; -band in active tiles)
-    uint32_t inside;         // every N5 lies in [-4096, 4096)^3 (origins -4096 or 0 on each axis)
+    uint32_t inside;         // bit 0: every N5 lies in [-4096, 4096)^3 (origins -4096 or 0 on each axis);
+                             // bit 1: some tile distance is 2^24 or more
     uint32_t n4, n3;         // node counts of the N4 and N3 pools (checked in bounds-checked builds)
 };
+
+// The N5 slot words of the box [-4096, 4096)^3 as one dense table of 64^3 words, which lies just
+// before slot5: word x << 12 | y << 6 | z for the N4-sized cell (x, y, z) of the box.
+constexpr uint32_t kTopWords = 64u * 64u * 64u;
 
 // One frame of one grid: the unit the persistent kernels draw ray tiles from.
 struct Job {
@@ -50,6 +55,8 @@ struct Tuning {
 };
 
 cudaError_t init_device_tables();
+// Fills the dense table before g.slot5 from the root block and slot5.
+cudaError_t build_top_table(const DevGrid &g, cudaStream_t st);
 int max_blocks_per_sm(int kernel, bool batched, int warps_per_block);
 // disjoint: the job's outputs do not overlap those of the previous kernel on st,
 // a k_pixel launch (see k_pixel); false is always safe.
