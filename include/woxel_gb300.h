@@ -162,9 +162,9 @@ int wx_grid_build(wx_ctx *ctx, wx_topology *topo, wx_grid **out);
 /* wx_grid_build with the SDF and the packing on the GPU (compute_sdf,
  * vdb345.rs:290-670): the same device pools word for word. Needs N5 origins
  * that are multiples of 4096 (else WX_ERR_UNSUPPORTED). Temporary device
- * memory: about 4 bytes per leaf voxel plus 200 bytes per node.
- * The sweeps hand containers to CTAs through a ready queue; a CTA whose
- * container is not ready polls for it, at most the context's SDF wait limit
+ * memory: about 460 bytes per leaf, 20 KB per N4 and 170 KB per N5.
+ * The distances are computed in steps, with a barrier of all CTAs between two
+ * steps; a CTA waiting there polls at most the context's SDF wait limit
  * (wx_ctx_set_sdf_wait_limit) times, then sets an error flag on which every
  * CTA returns: the call then returns WX_ERR_TIMEOUT, builds no grid and leaves
  * the context usable. */

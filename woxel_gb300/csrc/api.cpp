@@ -65,6 +65,7 @@ struct wx_grid {
     void *dev = nullptr;
     size_t bytes = 0;
     float *values = nullptr;  // level-set values (zero-crossing mode), own allocation
+    uint2 *ovf = nullptr;     // leaf overflow table where it is not part of dev
     wxk::DevGrid g{};
     wx_grid_info info{};
 };
@@ -312,6 +313,7 @@ void free_grid(wx_grid *gr) {
     if (!gr) return;
     cudaFree(gr->dev);
     if (gr->values) cudaFree(gr->values);
+    if (gr->ovf) cudaFree(gr->ovf);
     delete gr;
 }
 
@@ -718,97 +720,122 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
             return fail(ctx, WX_ERR_OOM, "wx_grid_build_gpu: host allocation failed");
         }
 
-        const uint64_t nmax = std::max<uint64_t>({n5, n4, n3, 1});
-        DevBuf kid5, val5, kid4, val4, val3, dpre5, dpre4, first4, first3, droot, c5, c4, org5, org4, org3, d5, d4, d3,
-            nb, indeg, queue, ctr;
-        struct Alloc {
-            DevBuf *b;
-            size_t bytes;
-        } allocs[] = {{&kid5, n5 * kN5Words * 8},  {&val5, n5 * kN5Words * 8}, {&kid4, n4 * kN4Words * 8},
-                      {&val4, n4 * kN4Words * 8},  {&val3, n3 * kN3Words * 8}, {&dpre5, n5 * kN5Words * 4},
-                      {&dpre4, n4 * kN4Words * 4}, {&first4, n5 * 4},          {&first3, n4 * 4},
-                      {&droot, root.size() * 16},  {&c5, n5 * kN5Slots * 4},   {&c4, n4 * kN4Slots * 4},
-                      {&org5, n5 * 16},            {&org4, n4 * 16},           {&org3, n3 * 16},
-                      {&d5, n5 * kN5Slots * 4},    {&d4, n4 * kN4Slots * 4},   {&d3, n3 * kN3Slots * 4},
-                      {&nb, nmax * 27 * 4},        {&indeg, nmax * 4},         {&queue, nmax * 4},
-                      {&ctr, 8 * 4}};
-        for (auto &a : allocs)
-            if (a.bytes) WX_CUDA(ctx, wx::dev_alloc(&a.b->p, a.bytes));
+        // Temporaries, carved from one allocation: masks, child tables, origins, neighbours and the sets of the
+        // distance computation.
+        DevBuf tmp;
+        size_t need = 0;
+        auto carve = [&](size_t bytes) {
+            const size_t at = need;
+            need += (bytes + 255) & ~(size_t)255;
+            return at;
+        };
+        const uint64_t nodes[3] = {n5, n4, n3}, words[3] = {n5 * kN5Words, n4 * kN4Words, n3 * kN3Words};
+        size_t z[3], val[2], f[3][2], w[3][2], org[3], nb[3], act[3], pre[2], first[2], cidx[2];
+        for (int l = 0; l < 3; l++) {
+            z[l] = carve(words[l] * 8);
+            for (int p = 0; p < 2; p++) {
+                f[l][p] = carve(words[l] * 8);
+                w[l][p] = carve(words[l] * 8);
+            }
+            org[l] = carve(nodes[l] * 16);
+            nb[l] = carve(nodes[l] * 27 * 4);
+            act[l] = carve(nodes[l] * 4);
+            if (l == 2) break;
+            val[l] = carve(words[l] * 8);
+            pre[l] = carve(words[l] * 4);
+            first[l] = carve(nodes[l] * 4);
+            cidx[l] = carve(words[l] * 64 * 4);
+        }
+        const size_t at_root = carve(root.size() * 16), at_ctl = carve(64);
+        WX_CUDA(ctx, wx::dev_alloc(&tmp.p, need));
+        char *const base = static_cast<char *>(tmp.p);
+        auto u64 = [&](size_t at) { return reinterpret_cast<uint64_t *>(base + at); };
+        auto u32 = [&](size_t at) { return reinterpret_cast<uint32_t *>(base + at); };
+        auto i4 = [&](size_t at) { return reinterpret_cast<int4 *>(base + at); };
+        // The grid's pools; the overflow table, rarely needed, follows in a block of its own.
+        wx_grid *gr = nullptr;
+        if ((rc = alloc_grid(ctx, o5, n5, n4, n3, 0, &gr)) != WX_OK) return rc;
+        struct Guard {
+            wx_grid *g;
+            ~Guard() { free_grid(g); }
+        } guard{gr};
         struct Up {
-            DevBuf *b;
+            size_t at;
             const void *src;
             size_t bytes;
-        } ups[] = {{&kid5, t->kid5.data(), n5 * kN5Words * 8}, {&val5, t->val5.data(), n5 * kN5Words * 8},
-                   {&kid4, t->kid4.data(), n4 * kN4Words * 8}, {&val4, t->val4.data(), n4 * kN4Words * 8},
-                   {&val3, t->val3.data(), n3 * kN3Words * 8}, {&dpre5, pre5.data(), n5 * kN5Words * 4},
-                   {&dpre4, pre4.data(), n4 * kN4Words * 4},   {&first4, t->first4.data(), n5 * 4},
-                   {&first3, t->first3.data(), n4 * 4},        {&droot, root.data(), root.size() * 16},
-                   {&org5, o5.data(), n5 * 16}};
+        } ups[] = {{z[0], t->kid5.data(), words[0] * 8},  {val[0], t->val5.data(), words[0] * 8},
+                   {z[1], t->kid4.data(), words[1] * 8},  {val[1], t->val4.data(), words[1] * 8},
+                   {z[2], t->val3.data(), words[2] * 8},  {pre[0], pre5.data(), words[0] * 4},
+                   {pre[1], pre4.data(), words[1] * 4},   {first[0], t->first4.data(), n5 * 4},
+                   {first[1], t->first3.data(), n4 * 4},  {at_root, root.data(), root.size() * 16},
+                   {org[0], o5.data(), n5 * 16}};
         for (auto &u : ups)
-            if (u.bytes) WX_CUDA(ctx, cudaMemcpy(u.b->p, u.src, u.bytes, cudaMemcpyHostToDevice));
+            if (u.bytes) WX_CUDA(ctx, cudaMemcpy(base + u.at, u.src, u.bytes, cudaMemcpyHostToDevice));
         const cudaStream_t st = nullptr;
-        WX_CUDA(ctx, cudaMemsetAsync(ctr.p, 0, 8 * 4, st));
-        WX_CUDA(ctx, wxk::sdf_child_table(kid5.as<uint64_t>(), dpre5.as<uint32_t>(), first4.as<uint32_t>(), n5, 15,
-                                          c5.as<uint32_t>(), st));
-        WX_CUDA(ctx, wxk::sdf_child_table(kid4.as<uint64_t>(), dpre4.as<uint32_t>(), first3.as<uint32_t>(), n4, 12,
-                                          c4.as<uint32_t>(), st));
-        WX_CUDA(ctx, wxk::sdf_child_origins(c5.as<uint32_t>(), org5.as<int4>(), n5, 5, 7, org4.as<int4>(), st));
-        WX_CUDA(ctx, wxk::sdf_child_origins(c4.as<uint32_t>(), org4.as<int4>(), n4, 4, 3, org3.as<int4>(), st));
-        WX_CUDA(ctx, wxk::sdf_init(kid5.as<uint64_t>(), n5 * kN5Slots, d5.as<uint32_t>(), st));
-        WX_CUDA(ctx, wxk::sdf_init(kid4.as<uint64_t>(), n4 * kN4Slots, d4.as<uint32_t>(), st));
-        WX_CUDA(ctx, wxk::sdf_init(val3.as<uint64_t>(), n3 * kN3Slots, d3.as<uint32_t>(), st));
-        const wxk::SdfTree tree{droot.as<int4>(), (uint32_t)n5, c5.as<uint32_t>(), c4.as<uint32_t>()};
-        struct Level {
-            int L;
-            DevBuf *org, *d;
-            uint64_t nc;
-        } levels[] = {{5, &org5, &d5, n5}, {4, &org4, &d4, n4}, {3, &org3, &d3, n3}};
-        for (auto &lv : levels) {
-            WX_CUDA(ctx, wxk::sdf_neighbours(lv.L, lv.org->as<int4>(), (uint32_t)lv.nc, tree, nb.as<uint32_t>(), st));
-            WX_CUDA(ctx, wxk::sdf_sweep(lv.L, lv.d->as<uint32_t>(), nb.as<uint32_t>(), (uint32_t)lv.nc,
-                                        indeg.as<uint32_t>(), queue.as<uint32_t>(), ctr.as<uint32_t>(), ctx->num_sms,
-                                        ctx->sdf_spins, st));
+        uint32_t *const ctl = u32(at_ctl);
+        auto *const left = reinterpret_cast<unsigned long long *>(base + at_ctl + 16);
+        WX_CUDA(ctx, cudaMemsetAsync(ctl, 0, 64, st));
+        if (n3) WX_CUDA(ctx, cudaMemsetAsync((void *)gr->g.leaf, 0, n3 * kN3Slots, st));
+        WX_CUDA(ctx, wxk::sdf_child_table(u64(z[0]), u32(pre[0]), u32(first[0]), n5, 15, u32(cidx[0]), st));
+        WX_CUDA(ctx, wxk::sdf_child_table(u64(z[1]), u32(pre[1]), u32(first[1]), n4, 12, u32(cidx[1]), st));
+        WX_CUDA(ctx, wxk::sdf_child_origins(u32(cidx[0]), i4(org[0]), n5, 5, 7, i4(org[1]), st));
+        WX_CUDA(ctx, wxk::sdf_child_origins(u32(cidx[1]), i4(org[1]), n4, 4, 3, i4(org[2]), st));
+        const wxk::SdfTree tree{i4(at_root), (uint32_t)n5, u32(cidx[0]), u32(cidx[1])};
+        uint32_t *const slots[2] = {const_cast<uint32_t *>(gr->g.slot5), const_cast<uint32_t *>(gr->g.slot4)};
+        wxk::SdfWork work{};
+        for (int l = 0; l < 3; l++) {
+            WX_CUDA(ctx, wxk::sdf_neighbours(5 - l, i4(org[l]), (uint32_t)nodes[l], tree, u32(nb[l]), st));
+            if (nodes[l]) {
+                WX_CUDA(ctx, cudaMemsetAsync(base + act[l], 0, nodes[l] * 4, st));
+                WX_CUDA(ctx, cudaMemcpyAsync(base + f[l][0], base + z[l], words[l] * 8, cudaMemcpyDeviceToDevice, st));
+                WX_CUDA(ctx, cudaMemcpyAsync(base + w[l][0], base + z[l], words[l] * 8, cudaMemcpyDeviceToDevice, st));
+            }
+            WX_CUDA(ctx, wxk::sdf_count_clear(u64(z[l]), words[l], left, st));
+            if (l == 2) {
+                WX_CUDA(ctx, wxk::sdf_count_clear(u64(z[l]), words[l], left + 2, st));
+                WX_CUDA(ctx, cudaMemcpyAsync(left + 1, left + 2, 8, cudaMemcpyDeviceToDevice, st));
+            } else WX_CUDA(ctx, wxk::sdf_pack_internal(u64(z[l]), u64(val[l]), u32(cidx[l]), words[l] * 64, slots[l], st));
+            work.lv[l] = wxk::SdfLevel{u64(z[l]),  l < 2 ? u64(val[l]) : nullptr, {u64(f[l][0]), u64(f[l][1])},
+                                       {u64(w[l][0]), u64(w[l][1])}, u32(nb[l]), u32(act[l]), l < 2 ? slots[l] : nullptr,
+                                       (uint32_t)nodes[l]};
         }
-        // Count the leaf overflow entries (ctr[3]) to size the grid block.
-        uint32_t *flags = ctr.as<uint32_t>();
-        WX_CUDA(ctx, wxk::sdf_pack_leaves(d3.as<uint32_t>(), n3 * kN3Slots, nullptr, nullptr, 0, flags + 3, st));
-        uint32_t h[8];
-        WX_CUDA(ctx, cudaMemcpy(h, flags, sizeof h, cudaMemcpyDeviceToHost));
-        if (h[2]) return fail(ctx, WX_ERR_TIMEOUT, "wx_grid_build_gpu: a sweep's dependency wait hit its bound");
-        const uint64_t n_ovf = h[3];
-        wx_grid *gr = nullptr;
-        if ((rc = alloc_grid(ctx, o5, n5, n4, n3, n_ovf, &gr)) != WX_OK) return rc;
-        cudaError_t e = cudaMemsetAsync(flags + 3, 0, 2 * 4, st);  // ctr[3] overflow count, ctr[4] distance error
-        if (e == cudaSuccess)
-            e = wxk::sdf_pack_internal(kid5.as<uint64_t>(), val5.as<uint64_t>(), c5.as<uint32_t>(), d5.as<uint32_t>(),
-                                       n5 * kN5Slots, const_cast<uint32_t *>(gr->g.slot5), flags + 4, st);
-        if (e == cudaSuccess)
-            e = wxk::sdf_pack_internal(kid4.as<uint64_t>(), val4.as<uint64_t>(), c4.as<uint32_t>(), d4.as<uint32_t>(),
-                                       n4 * kN4Slots, const_cast<uint32_t *>(gr->g.slot4), flags + 4, st);
-        if (e == cudaSuccess)
-            e = wxk::sdf_pack_leaves(d3.as<uint32_t>(), n3 * kN3Slots, const_cast<uint8_t *>(gr->g.leaf),
-                                     const_cast<uint2 *>(gr->g.ovf), (uint32_t)n_ovf, flags + 3, st);
-        if (e == cudaSuccess) e = wxk::build_top_table(gr->g, st);
-        if (e == cudaSuccess) e = cudaMemcpy(h, flags, sizeof h, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) {
-            free_grid(gr);
-            return cuda_fail(ctx, e, "wx_grid_build_gpu: packing");
-        }
-        if (h[4]) {
-            free_grid(gr);
-            return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build_gpu: tile distance >= 2^31");
-        }
-        if (n_ovf) {  // entries arrive in any order; the kernels binary-search them by key
-            std::vector<uint2> ov(n_ovf);
-            e = cudaMemcpy(ov.data(), gr->g.ovf, n_ovf * 8, cudaMemcpyDeviceToHost);
-            std::sort(ov.begin(), ov.end(), [](const uint2 &a, const uint2 &b) { return a.x < b.x; });
-            if (e == cudaSuccess) e = cudaMemcpy((void *)gr->g.ovf, ov.data(), n_ovf * 8, cudaMemcpyHostToDevice);
-            if (e != cudaSuccess) {
-                free_grid(gr);
-                return cuda_fail(ctx, e, "wx_grid_build_gpu: overflow table");
+        work.leaf = const_cast<uint8_t *>(gr->g.leaf);
+        work.ctl = ctl;
+        work.left = left;
+        // Distances below 255 first; the leaf cells then left are the overflow entries.
+        struct {
+            uint32_t ctl[4];
+            unsigned long long left[3];  // [2] the inactive leaf cells, as counted at the start
+        } h;
+        WX_CUDA(ctx, wxk::sdf_levels(work, 1, 254, ctx->num_sms, ctx->sdf_spins, st));
+        WX_CUDA(ctx, wxk::build_top_table(gr->g, st));
+        WX_CUDA(ctx, cudaMemcpy(&h, ctl, sizeof h, cudaMemcpyDeviceToHost));
+        if (!h.ctl[2] && h.left[0]) {
+            const uint64_t n_ovf = h.left[1];
+            if (n_ovf) {
+                if (n_ovf > UINT32_MAX) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build_gpu: overflow table");
+                WX_CUDA(ctx, wx::dev_alloc(&gr->ovf, n_ovf * 8));
+                gr->g.ovf = gr->ovf;
+                gr->g.n_ovf = (uint32_t)n_ovf;
+                gr->bytes += (n_ovf * 8 + 255) & ~(size_t)255;
+                gr->info.device_bytes = gr->bytes;
+            }
+            work.ovf = gr->ovf;
+            work.ovf_cap = (uint32_t)n_ovf;
+            WX_CUDA(ctx, wxk::sdf_levels(work, 255, wxk::kSdfMaxLevel, ctx->num_sms, ctx->sdf_spins, st));
+            WX_CUDA(ctx, wxk::build_top_table(gr->g, st));
+            WX_CUDA(ctx, cudaMemcpy(&h, ctl, sizeof h, cudaMemcpyDeviceToHost));
+            if (n_ovf && !h.ctl[2]) {  // entries arrive in any order; the kernels binary-search them by key
+                std::vector<uint2> ov(n_ovf);
+                WX_CUDA(ctx, cudaMemcpy(ov.data(), gr->ovf, n_ovf * 8, cudaMemcpyDeviceToHost));
+                std::sort(ov.begin(), ov.end(), [](const uint2 &a, const uint2 &b) { return a.x < b.x; });
+                WX_CUDA(ctx, cudaMemcpy(gr->ovf, ov.data(), n_ovf * 8, cudaMemcpyHostToDevice));
             }
         }
-        gr->info.active_voxels = wx_topology_active_voxels(t);
+        if (h.ctl[2]) return fail(ctx, WX_ERR_TIMEOUT, "wx_grid_build_gpu: the distance steps' barrier wait hit its bound");
+        if (h.left[0]) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build_gpu: distances above 4095");
+        gr->info.active_voxels = n3 * kN3Slots - h.left[2];
+        guard.g = nullptr;
         *out = gr;
         return WX_OK;
     });
@@ -932,6 +959,10 @@ int wx_grid_release(wx_ctx *ctx, wx_grid *grid) {
         cudaError_t e = cudaFree(grid->dev);
         if (grid->values) {
             const cudaError_t e2 = cudaFree(grid->values);
+            if (e == cudaSuccess) e = e2;
+        }
+        if (grid->ovf) {
+            const cudaError_t e2 = cudaFree(grid->ovf);
             if (e == cudaSuccess) e = e2;
         }
         delete grid;

@@ -88,18 +88,35 @@ cudaError_t sdf_child_table(const uint64_t *kid, const uint32_t *pre, const uint
                             int slots_log2, uint32_t *cidx, cudaStream_t st);
 cudaError_t sdf_child_origins(const uint32_t *cidx, const int4 *org, uint64_t nodes, int log2d, int child_span_log2,
                               int4 *org_child, cudaStream_t st);
-cudaError_t sdf_init(const uint64_t *solid, uint64_t ncells, uint32_t *d, cudaStream_t st);
 cudaError_t sdf_neighbours(int level, const int4 *org, uint32_t nc, const SdfTree &t, uint32_t *nb, cudaStream_t st);
-// Both passes of one level; ctr[2] (not reset here) is set when a wait hit its bound.
-// spin_limit: polls (256 ns apart) a CTA makes for its container before it sets
-// the error flag ctr[2] and every CTA of the sweep returns.
+// *count += the clear bits of `words` mask words.
+cudaError_t sdf_count_clear(const uint64_t *w, uint64_t words, unsigned long long *count, cudaStream_t st);
+// One level of the tree in the distance computation (sdf.cu). Masks are those of the grid (bit = cell, D^3 a node).
+struct SdfLevel {
+    const uint64_t *z;       // the cells that start at distance 0: children, active voxels
+    const uint64_t *val;     // N5/N4: active tiles
+    uint64_t *f[2], *w[2];   // forward and final sets, by the parity of k; set 0 starts as z
+    const uint32_t *nb;      // 27 neighbours of each node
+    uint32_t *act;           // last k at which the node or a neighbour changed; starts at 0
+    uint32_t *slot;          // N5/N4: slot words
+    uint32_t n;              // nodes
+};
+struct SdfWork {
+    SdfLevel lv[3];          // N5, N4, leaves
+    uint8_t *leaf;           // leaf bytes, 0 at the start
+    uint2 *ovf;              // (cell, distance) of distances >= 255
+    uint32_t ovf_cap;
+    uint32_t *ctl;           // 4 words: barrier arrivals and release, error flag, overflow entries
+    unsigned long long *left;  // cells without a distance: of all levels, of the leaves
+};
+// Steps k0..k1 (fewer when *left reaches 0). ctl[2] is set when a wait hit its bound.
+// spin_limit: polls (256 ns apart) a CTA makes at the barrier between two steps before it sets
+// the error flag and every CTA returns.
 constexpr uint32_t kSdfSpinLimit = 1u << 23;  // about 2 s
-cudaError_t sdf_sweep(int level, uint32_t *d, const uint32_t *nb, uint32_t nc, uint32_t *indeg, uint32_t *queue,
-                      uint32_t *ctr, int num_sms, uint32_t spin_limit, cudaStream_t st);
-cudaError_t sdf_pack_internal(const uint64_t *kid, const uint64_t *val, const uint32_t *cidx, const uint32_t *d,
-                              uint64_t nslots, uint32_t *slot, uint32_t *err, cudaStream_t st);
-cudaError_t sdf_pack_leaves(const uint32_t *d, uint64_t ncells, uint8_t *leaf, uint2 *ovf, uint32_t cap,
-                            uint32_t *n_ovf, cudaStream_t st);
+constexpr uint32_t kSdfMaxLevel = 4095u;      // no grid reaches it
+cudaError_t sdf_levels(const SdfWork &w, uint32_t k0, uint32_t k1, int num_sms, uint32_t spin_limit, cudaStream_t st);
+cudaError_t sdf_pack_internal(const uint64_t *kid, const uint64_t *val, const uint32_t *cidx, uint64_t nslots,
+                              uint32_t *slot, cudaStream_t st);
 
 // Exhaustive check of the fast floor-division path against IEEE division:
 // every divisor m < max_m and every significand of [1,2) and [-2,-1).
