@@ -27,9 +27,10 @@ using wxk::Job;
 // cp_main for one pixel of job J: colour, optional hit record, shadow ray (mode 3)
 // or the glossy chain (mode 4). Tile tl of the job covers tile_w x tile_h
 // pixels; lanes outside the dispatched region 8*floor(w/8) x 4*floor(h/4)
-// (wgpu_context.rs:281) do nothing. kAll = false compiles modes 0-3 only (the
-// host sends frames of modes 4 and 5 to the kAll = true kernels): the glossy
-// chain and the zero-crossing search would otherwise cost the march registers.
+// (wgpu_context.rs:281) do nothing. kModes: the modes compiled in (kBase 0-3,
+// kGlossy 4, kSurface 5; the host picks the kernel by the frames' modes): the
+// glossy chain and the zero-crossing search would otherwise cost the march
+// registers and instruction cache.
 // Pixel (gx, gy) of lane `lane` of tile tl; false outside the dispatched region.
 // Tile row: with order 1, the i-th row handed out is the middle row, then
 // alternately the rows above and below it (a permutation of the rows).
@@ -44,7 +45,9 @@ __device__ __forceinline__ bool tile_pixel(const Job &J, uint32_t tl, uint32_t l
     return gx < (J.width & ~7u) && gy < (J.height & ~3u);
 }
 
-template <bool kAll, bool kCompact = false>
+constexpr int kBase = 1, kGlossy = 2, kSurface = 4, kAllModes = 7;
+
+template <int kModes, bool kCompact = false>
 __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t lane, bool wait_prev) {
     uint32_t gx, gy;
     // The warp's lanes leave each march at different iterations. Without the
@@ -56,13 +59,25 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
     const wx_state_uniform &s = J.s;
     const F3 dir = primary_dir(s, gx, gy);
     const F3 eye = f3(s.eye[0], s.eye[1], s.eye[2]);
+    const uint32_t pix = gy * J.width + gx;
+    if ((kModes & kGlossy) && (kModes == kGlossy || s.render_mode[0] == 4u)) {
+        // The hit record is stored at the first hit, so that it is not live across the later rays.
+        const F3 c = glossy_colour(J.g, s, eye, dir, act, [&](const March &hit) {
+            if (!J.hits) return;
+            if (wait_prev) asm volatile("griddepcontrol.wait;" ::: "memory");
+            if (wx_in_range(pix, (uint64_t)J.width * J.height))
+                store_hit(J.hits + pix, hit.p, dot3(hit.p - eye, dir), hit.node,
+                          hit.state | (hit.np << 2) | (hit.mask << 4) | (hit.i << 8), 0u, 0u);
+        });
+        if (wait_prev) asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (wx_in_range(pix, (uint64_t)J.width * J.height)) J.rgba[pix] = pack_rgba(c);
+        return;
+    }
     const March hit = hdda(J.g, eye, dir);
     __syncwarp(act);
     F3 c;
     uint32_t shadow = 0, reserved = 0;
-    if (kAll && s.render_mode[0] == 4u) {
-        c = glossy_colour(J.g, s, hit, dir);
-    } else if (kAll && s.render_mode[0] == 5u) {  // zero crossing (extension); the mode is warp-uniform
+    if ((kModes & kSurface) && (kModes == kSurface || s.render_mode[0] == 5u)) {  // zero crossing (extension); the mode is warp-uniform
         reserved = 0x7FC00000u;           // NaN: no crossing
         if (hit.state == 0u) {
             float ts;
@@ -102,7 +117,6 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
             if (sh.state == 0u) cpk = pack_rgba(ambient_colour());  // shadowed is I_a
         }
         __syncwarp(act);
-        const uint32_t pix = gy * J.width + gx;
         if (wait_prev) asm volatile("griddepcontrol.wait;" ::: "memory");
         if (!wx_in_range(pix, (uint64_t)J.width * J.height)) return;
         J.rgba[pix] = cpk;
@@ -120,7 +134,6 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
         }
     }
     __syncwarp(act);
-    const uint32_t pix = gy * J.width + gx;
     // A programmatically dependent launch (k_pixel) may run its march while the
     // previous kernel of the stream finishes; unless that kernel's outputs are
     // disjoint from this frame's, the stores wait for it to complete. A no-op
@@ -137,11 +150,11 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
 // warp slots of an SM. Its march waits on dependent loads and leaves a third of its lanes idle, so
 // resident warps pay more than the five reloads an iteration that 32 registers cost: 8 frames of
 // 2000 spheres at 1080p take 3.27 ms at 32 registers, 3.47 at 40 and 3.67 at 47 (2 noise frames at
-// 4K: 2.20, 2.23 and 2.29 ms). Its kernel of every mode keeps 48 registers for the glossy and
-// zero-crossing code. The persistent kernels hold the job's pointers in registers and stay at 48
+// 4K: 2.20, 2.23 and 2.29 ms). The glossy kernel takes 0.38 ms for a 720p frame at 40 and 48
+// registers, 0.39 at 32 and 0.42 at 64; the zero-crossing kernel keeps 48. The persistent kernels hold the job's pointers in registers and stay at 48
 // (5 blocks, 40 warps): 48 mixed frames take 13.0 ms, 14.2 at 40 registers and 13.4 at 55.
 #define WX_RAY_BOUNDS __launch_bounds__(256, 5)
-#define WX_PIXEL_BOUNDS __launch_bounds__(256, kAll ? 5 : 8)
+#define WX_PIXEL_BOUNDS __launch_bounds__(256, kModes == kBase ? 8 : kModes == kGlossy ? 6 : 5)
 
 // One warp per tile of one frame, tiles in block order (rows in the job's order).
 // Frames on one stream overlap in time: the next k_pixel starts once every block
@@ -152,13 +165,13 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
 // host when this frame's outputs do not overlap that frame's) lets every block
 // write without waiting and retire as soon as its tiles are done, so the
 // previous frame's last blocks do not hold finished blocks on the SMs.
-template <bool kAll>
+template <int kModes>
 __global__ void WX_PIXEL_BOUNDS k_pixel(const __grid_constant__ Job job, uint32_t ntiles, uint32_t disjoint) {
     if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
     const uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (tile >= ntiles) return;
-    render_pixel<kAll>(job, tile, threadIdx.x & 31u, disjoint == 0u);
+    render_pixel<kModes>(job, tile, threadIdx.x & 31u, disjoint == 0u);
 }
 
 // ---------------------------------------------------------------------------
@@ -385,7 +398,7 @@ __device__ __forceinline__ uint32_t find_job(const Job *__restrict__ jobs, uint3
 // Batched launches may carry a cancel table (the server's): a job whose
 // cancel_id has been written to cancel[cancel_slot] (by the host, while the
 // launch runs) has its remaining tiles skipped, which `skipped` counts.
-template <bool kBatched, bool kAll>
+template <bool kBatched, int kModes>
 __global__ void WX_RAY_BOUNDS k_persistent(const Job *__restrict__ jobs, uint32_t njobs, const __grid_constant__ Job job0,
                              uint32_t total_tiles, uint32_t *__restrict__ ctr, const uint32_t *cancel,
                              uint32_t *skipped) {
@@ -410,9 +423,9 @@ __global__ void WX_RAY_BOUNDS k_persistent(const Job *__restrict__ jobs, uint32_
                     continue;
                 }
             }
-            render_pixel<kAll, true>(J, t - J.tile_begin + J.tile_off, lane, true);
+            render_pixel<kModes, true>(J, t - J.tile_begin + J.tile_off, lane, true);
         } else {
-            render_pixel<kAll, true>(job0, t, lane, true);
+            render_pixel<kModes, true>(job0, t, lane, true);
         }
     }
 }
@@ -484,8 +497,8 @@ cudaError_t build_top_table(const DevGrid &g, cudaStream_t st) {
 
 int max_blocks_per_sm(int kernel, bool batched, int warps_per_block) {
     const int threads = 32 * warps_per_block;
-    if (kernel == 1) return blocks_for(k_pixel<false>, threads);
-    return batched ? blocks_for(k_persistent<true, false>, threads) : blocks_for(k_persistent<false, false>, threads);
+    if (kernel == 1) return blocks_for(k_pixel<kBase>, threads);
+    return batched ? blocks_for(k_persistent<true, kBase>, threads) : blocks_for(k_persistent<false, kBase>, threads);
 }
 
 cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, cudaStream_t st) {
@@ -503,7 +516,8 @@ cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, cudaStr
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const uint32_t dj = disjoint ? 1u : 0u;
-    if (all_modes(job.s)) return cudaLaunchKernelEx(&cfg, k_pixel<true>, job, job.tiles, dj);
+    if (job.s.render_mode[0] == 4u) return cudaLaunchKernelEx(&cfg, k_pixel<kGlossy>, job, job.tiles, dj);
+    if (job.s.render_mode[0] == 5u) return cudaLaunchKernelEx(&cfg, k_pixel<kSurface>, job, job.tiles, dj);
     if (t.rays > 1) {  // k_wave: t.rays tiles per warp, lanes refill
         const uint32_t per_block = wpb * (uint32_t)t.rays;
         cfg.gridDim = dim3((job.tiles + per_block - 1) / per_block);
@@ -512,7 +526,7 @@ cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, cudaStr
         if (t.rays == 4) return cudaLaunchKernelEx(&cfg, k_wave<4>, job, job.tiles, dj);
         return cudaLaunchKernelEx(&cfg, k_wave<8>, job, job.tiles, dj);
     }
-    return cudaLaunchKernelEx(&cfg, k_pixel<false>, job, job.tiles, dj);
+    return cudaLaunchKernelEx(&cfg, k_pixel<kBase>, job, job.tiles, dj);
 }
 
 static int grid_blocks(const Tuning &t, bool batched, int num_sms, uint32_t total_tiles) {
@@ -528,10 +542,10 @@ cudaError_t launch_persistent(const Job &job, uint32_t *ctr, const Tuning &t, in
     if (e != cudaSuccess) return e;
     const int blocks = grid_blocks(t, false, num_sms, job.tiles);
     if (all_modes(job.s))
-        k_persistent<false, true><<<blocks, 32 * t.warps_per_block, 0, st>>>(nullptr, 1, job, job.tiles, ctr, nullptr,
+        k_persistent<false, kAllModes><<<blocks, 32 * t.warps_per_block, 0, st>>>(nullptr, 1, job, job.tiles, ctr, nullptr,
                                                                             nullptr);
     else
-        k_persistent<false, false><<<blocks, 32 * t.warps_per_block, 0, st>>>(nullptr, 1, job, job.tiles, ctr, nullptr,
+        k_persistent<false, kBase><<<blocks, 32 * t.warps_per_block, 0, st>>>(nullptr, 1, job, job.tiles, ctr, nullptr,
                                                                              nullptr);
     return cudaGetLastError();
 }
@@ -544,10 +558,10 @@ cudaError_t launch_batched(const Job *jobs_dev, uint32_t njobs, uint32_t total_t
     Job dummy{};
     const int blocks = grid_blocks(t, true, num_sms, total_tiles);
     if (all)
-        k_persistent<true, true><<<blocks, 32 * t.warps_per_block, 0, st>>>(jobs_dev, njobs, dummy, total_tiles, ctr,
+        k_persistent<true, kAllModes><<<blocks, 32 * t.warps_per_block, 0, st>>>(jobs_dev, njobs, dummy, total_tiles, ctr,
                                                                            cancel, skipped);
     else
-        k_persistent<true, false><<<blocks, 32 * t.warps_per_block, 0, st>>>(jobs_dev, njobs, dummy, total_tiles, ctr,
+        k_persistent<true, kBase><<<blocks, 32 * t.warps_per_block, 0, st>>>(jobs_dev, njobs, dummy, total_tiles, ctr,
                                                                             cancel, skipped);
     return cudaGetLastError();
 }

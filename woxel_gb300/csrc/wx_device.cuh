@@ -519,7 +519,7 @@ __device__ __forceinline__ F3 wall_colour(F3 N) {  // :300-305 / :333-338
     return r;
 }
 
-// Lit material colour shared by mode 4 and reflect_ray2/1 (:199-208, :280-290, :317-325).
+// Lit material colour of a hit in the glossy mode (:199-208, :280-290, :317-325).
 __device__ __forceinline__ F3 lit_colour(const DevGrid &g, const wx_state_uniform &s, const March &h, F3 step,
                                          F3 N) {
     const F3 sun = f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]);
@@ -532,30 +532,6 @@ __device__ __forceinline__ F3 lit_colour(const DevGrid &g, const wx_state_unifor
         if (hdda(g, src, -sun).state == 0u) return base + (I * sc) * 0.05f;
     }
     return base + I * sc;
-}
-
-__device__ __noinline__ F3 reflect_ray1(const DevGrid &g, const wx_state_uniform &s, F3 src, F3 dir) {  // :311-342
-    const March h = hdda(g, src, dir);
-    const F3 step = step3(dir);
-    if (h.state == 0u) return lit_colour(g, s, h, step, normalize3((-step) * maskf(h.mask)));
-    if (h.state == 1u) return wall_colour(normalize3((-step) * maskf(h.mask)));
-    return dir;
-}
-
-__device__ __noinline__ F3 reflect_ray2(const DevGrid &g, const wx_state_uniform &s, F3 src, F3 dir) {  // :267-309
-    const March h = hdda(g, src, dir);
-    const F3 step = step3(dir);
-    if (h.state == 0u) {
-        const F3 m = maskf(h.mask);
-        const F3 N = normalize3((-step) * m);
-        const F3 rdir = normalize3(dir - (2.0f * N) * dot3(dir, N));
-        const F3 rsrc = h.p - (4e-2f * step) * m;
-        const F3 rcol = reflect_ray1(g, s, rsrc, rdir);
-        const F3 mcol = lit_colour(g, s, h, step, N);
-        return mix3(mcol, rcol, kReflect);
-    }
-    if (h.state == 1u) return wall_colour(normalize3((-step) * maskf(h.mask)));
-    return dir;
 }
 
 __device__ __forceinline__ bool grid_line(float f, float m) { return fmodf(f, m) == 0.0f; }
@@ -623,32 +599,55 @@ __device__ __forceinline__ F3 primary_colour(const wx_state_uniform &s, const Ma
     return dir;
 }
 
-// Glossy mode (:195-224 for state 0, :246-257 for state 1), up to six rays.
-__device__ __noinline__ F3 glossy_colour(const DevGrid &g, const wx_state_uniform &s, const March &hit, F3 dir) {
-    const F3 step = step3(dir);
-    const F3 m = maskf(hit.mask);
-    const F3 N = normalize3((-step) * m);
-    if (hit.state == 0u) {
-        const F3 mcol = lit_colour(g, s, hit, step, N);
-        const F3 rdir = normalize3(dir - (2.0f * N) * dot3(dir, N));
-        const F3 rsrc = hit.p - (4e-2f * step) * m;
-        const F3 rcol = reflect_ray2(g, s, rsrc, rdir);
-        return mix3(mcol, rcol, kReflect);
+// Colour of a primary ray of the glossy mode that left the grid (:246-257).
+__device__ __forceinline__ F3 glossy_wall(F3 N, float py) {
+    const F3 Np = f3(pmax(0.0f, N.x), pmax(0.0f, N.y), pmax(0.0f, N.z));
+    const F3 Nn = -f3(pmin(0.0f, N.x), pmin(0.0f, N.y), pmin(0.0f, N.z));
+    const float ty = __fdiv_rn(py, 4096.0f);
+    const float w1 = kWall * 0.1f;
+    F3 r = mix3(f3(kWall, 0.0f, 0.0f), f3(w1, 0.0f, 0.0f), ty) * Np.x;
+    r = r + f3(0.0f, kWall, 0.0f) * Np.y;
+    r = r + mix3(f3(0.0f, 0.0f, kWall), f3(0.0f, 0.0f, w1), ty) * Np.z;
+    r = r + mix3(f3(kWall, kWall, 0.0f), f3(w1, w1, 0.0f), ty) * Nn.x;
+    r = r + f3(0.0f, kWall, kWall) * Nn.y;
+    r = r + mix3(f3(kWall, 0.0f, kWall), f3(w1, 0.0f, w1), ty) * Nn.z;
+    return r;
+}
+
+// The glossy mode (:195-224, :246-257, reflect_ray2 :267-309, reflect_ray1 :311-342): the primary ray and up to two
+// reflections, each hit with a shadow ray. One loop over the depth, so the march is in the code twice (camera or
+// reflected ray, shadow ray) and the warp's rays of one depth start together: as six inlined marches in nested calls
+// the kernel waited for instructions (6.0 of 15 stall cycles an issue) at 14 of 32 lanes. act: the warp's lanes that
+// are here; first(hit) is called once with the primary ray's result.
+template <class First>
+__device__ __forceinline__ F3 glossy_colour(const DevGrid &g, const wx_state_uniform &s, F3 src, F3 dir, uint32_t act,
+                                            First first) {
+    F3 c, m0, m1;
+    m0 = m1 = splat(0.0f);
+    uint32_t depth = 0;
+#pragma unroll 1
+    for (;; depth++) {
+        const March hit = hdda(g, src, dir);
+        if (depth == 0u) first(hit);
+        const bool lit = hit.state == 0u;
+        act = __ballot_sync(act, lit);
+        const F3 step = step3(dir), m = maskf(hit.mask);
+        const F3 N = normalize3((-step) * m);
+        if (!lit) {
+            c = hit.state == 1u ? (depth == 0u ? glossy_wall(N, hit.p.y) : wall_colour(N)) : dir;
+            break;
+        }
+        c = lit_colour(g, s, hit, step, N);
+        if (depth == 2u) break;
+        if (depth == 0u) m0 = c;
+        else m1 = c;
+        dir = normalize3(dir - (2.0f * N) * dot3(dir, N));
+        src = hit.p - (4e-2f * step) * m;
+        __syncwarp(act);
     }
-    if (hit.state == 1u) {
-        const F3 Np = f3(pmax(0.0f, N.x), pmax(0.0f, N.y), pmax(0.0f, N.z));
-        const F3 Nn = -f3(pmin(0.0f, N.x), pmin(0.0f, N.y), pmin(0.0f, N.z));
-        const float ty = __fdiv_rn(hit.p.y, 4096.0f);
-        const float w1 = kWall * 0.1f;
-        F3 r = mix3(f3(kWall, 0.0f, 0.0f), f3(w1, 0.0f, 0.0f), ty) * Np.x;
-        r = r + f3(0.0f, kWall, 0.0f) * Np.y;
-        r = r + mix3(f3(0.0f, 0.0f, kWall), f3(0.0f, 0.0f, w1), ty) * Np.z;
-        r = r + mix3(f3(kWall, kWall, 0.0f), f3(w1, w1, 0.0f), ty) * Nn.x;
-        r = r + f3(0.0f, kWall, kWall) * Nn.y;
-        r = r + mix3(f3(kWall, 0.0f, kWall), f3(w1, 0.0f, w1), ty) * Nn.z;
-        return r;
-    }
-    return dir;
+    if (depth == 2u) c = mix3(m1, c, kReflect);
+    if (depth >= 1u) c = mix3(m0, c, kReflect);
+    return c;
 }
 
 // cp_main's ray (raycast.comp.wgsl:62-63) for pixel (gx, gy).
