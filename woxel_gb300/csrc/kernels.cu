@@ -151,10 +151,11 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
 // resident warps pay more than the five reloads an iteration that 32 registers cost: 8 frames of
 // 2000 spheres at 1080p take 3.27 ms at 32 registers, 3.47 at 40 and 3.67 at 47 (2 noise frames at
 // 4K: 2.20, 2.23 and 2.29 ms). The glossy kernel takes 0.38 ms for a 720p frame at 40 and 48
-// registers, 0.39 at 32 and 0.42 at 64; the zero-crossing kernel keeps 48. The persistent kernels hold the job's pointers in registers and stay at 48
+// registers, 0.39 at 32 and 0.42 at 64; a zero-crossing 1080p frame 0.54 ms at 32, 0.58 at 40 and 0.59
+// at 48. The persistent kernels hold the job's pointers in registers and stay at 48
 // (5 blocks, 40 warps): 48 mixed frames take 13.0 ms, 14.2 at 40 registers and 13.4 at 55.
 #define WX_RAY_BOUNDS __launch_bounds__(256, 5)
-#define WX_PIXEL_BOUNDS __launch_bounds__(256, kModes == kBase ? 8 : kModes == kGlossy ? 6 : 5)
+#define WX_PIXEL_BOUNDS __launch_bounds__(256, kModes == kGlossy ? 6 : 8)
 
 // One warp per tile of one frame, tiles in block order (rows in the job's order).
 // Frames on one stream overlap in time: the next k_pixel starts once every block
