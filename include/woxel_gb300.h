@@ -154,7 +154,9 @@ int wx_ctx_destroy(wx_ctx *ctx);
 const char *wx_last_error(const wx_ctx *ctx);
 
 /* ---- grids: replace the atlas/mask upload (wgpu_context.rs:101-159, 506-573) ---- */
-/* Drop-in: repack the Rust side's flattened view into device node pools. */
+/* Drop-in: repack the Rust side's flattened view into device node pools. The
+ * atlases are copied and packed in pieces: temporary device memory is the masks
+ * and at most 256 MB (or one layer of nodes of an atlas, if that is more). */
 int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *view, wx_grid **out);
 /* Native: compute the per-level SDF (vdb345.rs:290-670) on the host and pack
  * the pools directly from a topology, without the padded atlas. */

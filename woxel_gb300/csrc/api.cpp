@@ -192,22 +192,6 @@ struct DevBuf {
     }
 };
 
-template <class F>
-void parallel_chunks(size_t n, F f) {
-    unsigned nt = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    if (n < 4096 || nt == 1) {
-        f(0, n);
-        return;
-    }
-    std::vector<std::thread> th;
-    const size_t chunk = (n + nt - 1) / nt;
-    for (unsigned t = 0; t < nt; t++) {
-        const size_t lo = t * chunk, hi = std::min(n, lo + chunk);
-        if (lo < hi) th.emplace_back([=] { f(lo, hi); });
-    }
-    for (auto &x : th) x.join();
-}
-
 // The root block: header, origins and the dense table of root keys, which
 // replaces the linear scan of get_vdb_leaf_from_nothing
 // (raycast.comp.wgsl:398-413) with one load. The scan compares
@@ -317,12 +301,37 @@ void free_grid(wx_grid *gr) {
     delete gr;
 }
 
+// Frees a grid under construction on scope exit.
+struct GridGuard {
+    wx_grid *g;
+    ~GridGuard() { free_grid(g); }
+};
+
+// The leaf overflow table of n entries in a block of its own, for builds that learn n after alloc_grid.
+int alloc_overflow(wx_ctx *ctx, wx_grid *gr, uint64_t n) {
+    if (n > UINT32_MAX) return fail(ctx, WX_ERR_UNSUPPORTED, "leaf overflow table of 2^32 entries or more");
+    WX_CUDA(ctx, wx::dev_alloc(&gr->ovf, n * 8));
+    gr->g.ovf = gr->ovf;
+    gr->g.n_ovf = (uint32_t)n;
+    gr->bytes += (n * 8 + 255) & ~(size_t)255;
+    gr->info.device_bytes = gr->bytes;
+    return WX_OK;
+}
+
+// The kernels list overflow entries in any order; the march binary-searches them by key.
+int sort_overflow(wx_ctx *ctx, wx_grid *gr) {
+    std::vector<uint2> ov(gr->g.n_ovf);
+    WX_CUDA(ctx, cudaMemcpy(ov.data(), gr->ovf, ov.size() * 8, cudaMemcpyDeviceToHost));
+    std::sort(ov.begin(), ov.end(), [](const uint2 &a, const uint2 &b) { return a.x < b.x; });
+    WX_CUDA(ctx, cudaMemcpy(gr->ovf, ov.data(), ov.size() * 8, cudaMemcpyHostToDevice));
+    return WX_OK;
+}
+
 // Pack the per-voxel u32 leaf distances into bytes plus the overflow table,
-// allocate one device block for all pools and upload them. far_tiles: some N5 or N4 distance is
-// 2^24 or more (a hand-made view; compute_sdf's stay below 2000, the side of the largest cube of
-// nodes that a grid can hold).
+// allocate one device block for all pools and upload them. The distances are
+// compute_sdf's, far below 2^24 (the side of the largest cube of nodes that a grid can hold).
 int upload_pools(wx_ctx *ctx, const std::vector<int4> &o5, const uint32_t *s5, const uint32_t *s4, const uint32_t *s3,
-                 uint64_t n5, uint64_t n4, uint64_t n3, bool far_tiles, wx_grid **out) {
+                 uint64_t n5, uint64_t n4, uint64_t n3, wx_grid **out) {
     int rc = check_pool_limits(ctx, n5, n4, n3);
     if (rc != WX_OK) return rc;
     std::vector<uint8_t> leaf;
@@ -356,7 +365,6 @@ int upload_pools(wx_ctx *ctx, const std::vector<int4> &o5, const uint32_t *s5, c
     if (e == cudaSuccess && n3) e = cudaMemcpy((void *)gr->g.leaf, leaf.data(), leaf.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !ovf.empty())
         e = cudaMemcpy((void *)gr->g.ovf, ovf.data(), ovf.size() * 8, cudaMemcpyHostToDevice);
-    if (far_tiles) gr->g.inside |= 2u;
     if (e == cudaSuccess) e = wxk::build_top_table(gr->g, nullptr);
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
     if (e != cudaSuccess) {
@@ -665,7 +673,7 @@ int wx_grid_build(wx_ctx *ctx, wx_topology *t, wx_grid **out) {
         }
         if (too_far) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build: tile distance >= 2^31");
         wx_grid *gr = nullptr;
-        rc = upload_pools(ctx, o5, s5.data(), s4.data(), t->slot3.data(), n5, n4, n3, false, &gr);
+        rc = upload_pools(ctx, o5, s5.data(), s4.data(), t->slot3.data(), n5, n4, n3, &gr);
         if (rc != WX_OK) return rc;
         gr->info.active_voxels = wx_topology_active_voxels(t);
         *out = gr;
@@ -755,10 +763,7 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
         // The grid's pools; the overflow table, rarely needed, follows in a block of its own.
         wx_grid *gr = nullptr;
         if ((rc = alloc_grid(ctx, o5, n5, n4, n3, 0, &gr)) != WX_OK) return rc;
-        struct Guard {
-            wx_grid *g;
-            ~Guard() { free_grid(g); }
-        } guard{gr};
+        GridGuard guard{gr};
         struct Up {
             size_t at;
             const void *src;
@@ -812,25 +817,13 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
         WX_CUDA(ctx, cudaMemcpy(&h, ctl, sizeof h, cudaMemcpyDeviceToHost));
         if (!h.ctl[2] && h.left[0]) {
             const uint64_t n_ovf = h.left[1];
-            if (n_ovf) {
-                if (n_ovf > UINT32_MAX) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build_gpu: overflow table");
-                WX_CUDA(ctx, wx::dev_alloc(&gr->ovf, n_ovf * 8));
-                gr->g.ovf = gr->ovf;
-                gr->g.n_ovf = (uint32_t)n_ovf;
-                gr->bytes += (n_ovf * 8 + 255) & ~(size_t)255;
-                gr->info.device_bytes = gr->bytes;
-            }
+            if (n_ovf && (rc = alloc_overflow(ctx, gr, n_ovf)) != WX_OK) return rc;
             work.ovf = gr->ovf;
             work.ovf_cap = (uint32_t)n_ovf;
             WX_CUDA(ctx, wxk::sdf_levels(work, 255, wxk::kSdfMaxLevel, ctx->num_sms, ctx->sdf_spins, st));
             WX_CUDA(ctx, wxk::build_top_table(gr->g, st));
             WX_CUDA(ctx, cudaMemcpy(&h, ctl, sizeof h, cudaMemcpyDeviceToHost));
-            if (n_ovf && !h.ctl[2]) {  // entries arrive in any order; the kernels binary-search them by key
-                std::vector<uint2> ov(n_ovf);
-                WX_CUDA(ctx, cudaMemcpy(ov.data(), gr->ovf, n_ovf * 8, cudaMemcpyDeviceToHost));
-                std::sort(ov.begin(), ov.end(), [](const uint2 &a, const uint2 &b) { return a.x < b.x; });
-                WX_CUDA(ctx, cudaMemcpy(gr->ovf, ov.data(), n_ovf * 8, cudaMemcpyHostToDevice));
-            }
+            if (n_ovf && !h.ctl[2] && (rc = sort_overflow(ctx, gr)) != WX_OK) return rc;
         }
         if (h.ctl[2]) return fail(ctx, WX_ERR_TIMEOUT, "wx_grid_build_gpu: the distance steps' barrier wait hit its bound");
         if (h.left[0]) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build_gpu: distances above 4095");
@@ -881,72 +874,90 @@ int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *v, wx_grid **out) {
         };
         if (!block_ok(0, n5, d5, 32) || !block_ok(1, n4, d4, 16) || !block_ok(2, n3, d3, 8))
             return fail(ctx, WX_ERR_INVALID, "wx_grid_upload: atlas dimensions too small for the node counts");
-        auto texel = [&](int lvl, uint64_t idx, uint32_t d, uint32_t nd, uint32_t cx, uint32_t cy, uint32_t cz) {
-            const uint64_t x = nd * (idx % d) + cx, y = nd * ((idx / d) % d) + cy, z = nd * (idx / ((uint64_t)d * d)) + cz;
-            return v->atlas[lvl][(z * v->dims[lvl][1] + y) * v->dims[lvl][0] + x];
-        };
-        std::vector<uint32_t> s5, s4, s3;
+        int rc = check_pool_limits(ctx, n5, n4, n3);
+        if (rc != WX_OK) return rc;
         std::vector<int4> o5(std::max<uint64_t>(n5, 1));
-        try {
-            s5.resize(n5 * wx::kN5Slots);
-            s4.resize(n4 * wx::kN4Slots);
-            s3.resize(n3 * wx::kN3Slots);
-        } catch (...) {
-            return fail(ctx, WX_ERR_OOM, "wx_grid_upload: host allocation failed");
-        }
-        std::atomic<int> bad{0};
-        std::atomic<bool> far{false};
         for (uint64_t i = 0; i < n5; i++) {
             const int32_t *o = v->origins + i * v->origin_stride;
             o5[i] = make_int4(o[0], o[1], o[2], 0);
         }
-        parallel_chunks(n5, [&](size_t lo, size_t hi) {
-            for (size_t i = lo; i < hi; i++)
-                for (uint32_t s = 0; s < wx::kN5Slots; s++) {
-                    const uint32_t w = s >> 5, b = 1u << (s & 31);
-                    const bool kid = v->kids5[i * 1024 + w] & b, val = v->vals5[i * 1024 + w] & b;
-                    uint32_t c[3];
-                    wx::offset_child(s, 5, c);
-                    const uint32_t tx = texel(0, i, d5, 32, c[0], c[1], c[2]);
-                    uint32_t word;
-                    if (val) word = 0;
-                    else if (kid) { word = wx::kChildFlag | tx; if (tx >= n4) bad = 1; }
-                    else { word = tx; if (tx >= wx::kChildFlag) bad = 2; else if (tx >= (1u << 24)) far = true; }
-                    s5[i * wx::kN5Slots + s] = word;
-                }
-        });
-        parallel_chunks(n4, [&](size_t lo, size_t hi) {
-            for (size_t j = lo; j < hi; j++)
-                for (uint32_t s = 0; s < wx::kN4Slots; s++) {
-                    const uint32_t w = s >> 5, b = 1u << (s & 31);
-                    const bool kid = v->kids4[j * 128 + w] & b, val = v->vals4[j * 128 + w] & b;
-                    uint32_t c[3];
-                    wx::offset_child(s, 4, c);
-                    const uint32_t tx = texel(1, j, d4, 16, c[0], c[1], c[2]);
-                    uint32_t word;
-                    if (val) word = 0;
-                    else if (kid) { word = wx::kChildFlag | tx; if (tx >= n3) bad = 1; }
-                    else { word = tx; if (tx >= wx::kChildFlag) bad = 2; else if (tx >= (1u << 24)) far = true; }
-                    s4[j * wx::kN4Slots + s] = word;
-                }
-        });
-        parallel_chunks(n3, [&](size_t lo, size_t hi) {
-            for (size_t k = lo; k < hi; k++)
-                for (uint32_t s = 0; s < wx::kN3Slots; s++) {
-                    const bool val = v->vals3[k * 16 + (s >> 5)] & (1u << (s & 31));
-                    uint32_t c[3];
-                    wx::offset_child(s, 3, c);
-                    s3[k * wx::kN3Slots + s] = val ? 0u : texel(2, k, d3, 8, c[0], c[1], c[2]);
-                }
-        });
-        if (bad == 1) return fail(ctx, WX_ERR_INVALID, "wx_grid_upload: child index in atlas out of range");
-        if (bad == 2) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_upload: internal tile distance >= 2^31");
+        // The masks and, slab by slab, the atlases are copied to the device and packed there (pack.cu). A slab is a
+        // layer of d * d nodes (D texel layers, contiguous); the buffer holds as many as fit 256 MB, at least one.
+        struct Atlas {
+            int level;
+            uint64_t n, layers, per_buffer;
+            uint32_t d;
+            size_t layer_bytes;
+        } atlas[3] = {{5, n5, 0, 0, d5, 0}, {4, n4, 0, 0, d4, 0}, {3, n3, 0, 0, d3, 0}};
+        size_t slab = 0;
+        for (int l = 0; l < 3; l++) {
+            Atlas &a = atlas[l];
+            if (!a.n) continue;
+            const uint64_t per = (uint64_t)a.d * a.d;
+            a.layers = (a.n + per - 1) / per;
+            a.layer_bytes = ((size_t)v->dims[l][0] * v->dims[l][1] << a.level) * 4;
+            a.per_buffer = std::min<uint64_t>(a.layers, std::max<uint64_t>(1, ((size_t)256 << 20) / a.layer_bytes));
+            slab = std::max(slab, (size_t)a.per_buffer * a.layer_bytes);
+        }
+        const size_t words[5] = {n5 * 1024, n5 * 1024, n4 * 128, n4 * 128, n3 * 16};
+        const uint32_t *const src[5] = {v->kids5, v->vals5, v->kids4, v->vals4, v->vals3};
+        size_t at[5], need = 256;  // 256 bytes of counters
+        for (int i = 0; i < 5; i++) {
+            at[i] = need;
+            need += (words[i] * 4 + 255) & ~(size_t)255;
+        }
+        DevBuf tmp;
+        WX_CUDA(ctx, wx::dev_alloc(&tmp.p, need + slab));
+        char *const base = static_cast<char *>(tmp.p);
+        const uint32_t *mask[5];
+        for (int i = 0; i < 5; i++) {
+            mask[i] = reinterpret_cast<const uint32_t *>(base + at[i]);
+            if (words[i]) WX_CUDA(ctx, cudaMemcpy(base + at[i], src[i], words[i] * 4, cudaMemcpyHostToDevice));
+        }
         wx_grid *gr = nullptr;
-        int rc = upload_pools(ctx, o5, s5.data(), s4.data(), s3.data(), n5, n4, n3, far, &gr);
-        if (rc != WX_OK) return rc;
-        uint64_t act = 0;
-        for (uint64_t w = 0; w < n3 * 16; w++) act += (uint64_t)__builtin_popcount(v->vals3[w]);
-        gr->info.active_voxels = act;
+        if ((rc = alloc_grid(ctx, o5, n5, n4, n3, 0, &gr)) != WX_OK) return rc;
+        GridGuard guard{gr};
+        const cudaStream_t st = nullptr;
+        struct Counts {
+            unsigned long long n_ovf, clear;
+            uint32_t flags;
+        } h{}, *const dev = reinterpret_cast<Counts *>(base);
+        WX_CUDA(ctx, cudaMemsetAsync(dev, 0, sizeof(Counts), st));
+        auto pack = [&](int l) -> cudaError_t {
+            const Atlas &a = atlas[l];
+            for (uint64_t z = 0; z < a.layers; z += a.per_buffer) {
+                const uint64_t nz = std::min(a.per_buffer, a.layers - z), per = (uint64_t)a.d * a.d;
+                const char *from = reinterpret_cast<const char *>(v->atlas[l]) + z * a.layer_bytes;
+                cudaError_t e = cudaMemcpy(base + need, from, nz * a.layer_bytes, cudaMemcpyHostToDevice);
+                if (e != cudaSuccess) return e;
+                const wxk::ViewSlab s{reinterpret_cast<const uint32_t *>(base + need), v->dims[l][0], v->dims[l][1], a.d,
+                                      z * per, std::min(nz * per, a.n - z * per)};
+                if (l < 2)
+                    e = wxk::pack_view_nodes(a.level, s, mask[2 * l], mask[2 * l + 1], (uint32_t)(l == 0 ? n4 : n3),
+                                             const_cast<uint32_t *>(l == 0 ? gr->g.slot5 : gr->g.slot4), &dev->flags, st);
+                else
+                    e = wxk::pack_view_leaves(s, mask[4], const_cast<uint8_t *>(gr->g.leaf), gr->ovf, gr->g.n_ovf,
+                                              &dev->n_ovf, st);
+                if (e != cudaSuccess) return e;
+            }
+            return cudaSuccess;
+        };
+        for (int l = 0; l < 3; l++) WX_CUDA(ctx, pack(l));
+        WX_CUDA(ctx, wxk::sdf_count_clear(reinterpret_cast<const uint64_t *>(mask[4]), n3 * 8, &dev->clear, st));
+        WX_CUDA(ctx, wxk::build_top_table(gr->g, st));
+        WX_CUDA(ctx, cudaMemcpy(&h, dev, sizeof h, cudaMemcpyDeviceToHost));
+        if (h.flags & 1u) return fail(ctx, WX_ERR_INVALID, "wx_grid_upload: child index in atlas out of range");
+        if (h.flags & 2u) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_upload: internal tile distance >= 2^31");
+        if (h.flags & 4u) gr->g.inside |= 2u;
+        if (h.n_ovf) {  // rare (hand-made views): the leaves once more, now with the overflow table
+            rc = alloc_overflow(ctx, gr, h.n_ovf);
+            if (rc != WX_OK) return rc;
+            WX_CUDA(ctx, cudaMemsetAsync(dev, 0, sizeof(Counts), st));
+            WX_CUDA(ctx, pack(2));
+            if ((rc = sort_overflow(ctx, gr)) != WX_OK) return rc;
+        }
+        gr->info.active_voxels = n3 * wx::kN3Slots - h.clear;
+        guard.g = nullptr;
         *out = gr;
         return WX_OK;
     });

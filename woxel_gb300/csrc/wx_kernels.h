@@ -118,6 +118,20 @@ cudaError_t sdf_levels(const SdfWork &w, uint32_t k0, uint32_t k1, int num_sms, 
 cudaError_t sdf_pack_internal(const uint64_t *kid, const uint64_t *val, const uint32_t *cidx, uint64_t nslots,
                               uint32_t *slot, cudaStream_t st);
 
+// Packing of the flattened view (pack.cu): z slabs of an atlas in device memory, as block rows of nodes. The
+// texel of node idx's slot (x, y, z) is at ((idx' / d^2 * D + z) * h + (idx' / d % d * D + y)) * w + idx' % d * D + x
+// with idx' = idx - first.
+struct ViewSlab {
+    const uint32_t *texels;
+    uint32_t w, h;       // texture width and height
+    uint32_t d;          // nodes per row and rows per layer, as the shader derives them
+    uint64_t first, count;  // nodes of the slab
+};
+cudaError_t pack_view_nodes(int level, const ViewSlab &s, const uint32_t *kids, const uint32_t *vals, uint32_t nchild,
+                            uint32_t *slot, uint32_t *flags, cudaStream_t st);
+cudaError_t pack_view_leaves(const ViewSlab &s, const uint32_t *vals, uint8_t *leaf, uint2 *ovf, uint32_t cap,
+                             unsigned long long *n_ovf, cudaStream_t st);
+
 // Exhaustive check of the fast floor-division path against IEEE division:
 // every divisor m < max_m and every significand of [1,2) and [-2,-1).
 // out[0] = mismatch count, out[1] = first mismatching m, out[2] = its x bits.
