@@ -682,9 +682,9 @@ int wx_grid_build(wx_ctx *ctx, wx_topology *t, wx_grid **out) {
 }
 
 // The same pools as wx_grid_build, with compute_sdf and the packing on the
-// GPU (sdf.cu). The host uploads only the masks, the N5 origins and per-word
-// child-count prefixes; child tables, child origins, neighbour tables, the
-// three sweeps and the packing run on the device.
+// GPU (sdf.cu). The host uploads only the masks and the N5 origins; child
+// tables, child origins, neighbour tables, the distances and the packing run on
+// the device.
 int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
     return wx::guard("wx_grid_build_gpu", [&]() -> int {
         if (!ctx || !t || !out) return fail(ctx, WX_ERR_INVALID, "wx_grid_build_gpu: null argument");
@@ -698,29 +698,11 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
             t->first3.size() != n4)
             return fail(ctx, WX_ERR_INVALID, "wx_grid_build_gpu: masks and node counts disagree");
         std::vector<int4> o5(std::max<uint64_t>(n5, 1));
-        std::vector<uint32_t> pre5, pre4;
-        try {
-            pre5.resize(n5 * kN5Words);
-            pre4.resize(n4 * kN4Words);
-        } catch (...) {
-            return fail(ctx, WX_ERR_OOM, "wx_grid_build_gpu: host allocation failed");
-        }
         for (uint64_t i = 0; i < n5; i++) {
             o5[i] = make_int4(t->o5[i][0], t->o5[i][1], t->o5[i][2], 0);
             if ((o5[i].x & 4095) || (o5[i].y & 4095) || (o5[i].z & 4095))
                 return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build_gpu: N5 origins must be multiples of 4096");
         }
-        auto prefix = [](const std::vector<uint64_t> &kid, uint64_t nodes, uint32_t words, std::vector<uint32_t> &pre) {
-            for (uint64_t n = 0; n < nodes; n++) {
-                uint32_t acc = 0;
-                for (uint32_t w = 0; w < words; w++) {
-                    pre[n * words + w] = acc;
-                    acc += (uint32_t)__builtin_popcountll(kid[n * words + w]);
-                }
-            }
-        };
-        prefix(t->kid5, n5, kN5Words, pre5);
-        prefix(t->kid4, n4, kN4Words, pre4);
         std::vector<int4> root;
         try {
             root = root_block(o5, n5);
@@ -738,16 +720,13 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
             return at;
         };
         const uint64_t nodes[3] = {n5, n4, n3}, words[3] = {n5 * kN5Words, n4 * kN4Words, n3 * kN3Words};
-        size_t z[3], val[2], f[3][2], w[3][2], org[3], nb[3], act[3], pre[2], first[2], cidx[2];
+        size_t z[3], val[2], org[3], nb[3], act[3], pre[2], first[2], cidx[2];
+        const uint64_t node_words[3] = {kN5Words, kN4Words, kN3Words};
         for (int l = 0; l < 3; l++) {
-            z[l] = carve(words[l] * 8);
-            for (int p = 0; p < 2; p++) {
-                f[l][p] = carve(words[l] * 8);
-                w[l][p] = carve(words[l] * 8);
-            }
+            z[l] = carve((words[l] + node_words[l]) * (wxk::kSdfWindow + 3) * 8);
             org[l] = carve(nodes[l] * 16);
             nb[l] = carve(nodes[l] * 27 * 4);
-            act[l] = carve(nodes[l] * 4);
+            act[l] = carve((nodes[l] + 1) * 4);
             if (l == 2) break;
             val[l] = carve(words[l] * 8);
             pre[l] = carve(words[l] * 4);
@@ -770,17 +749,15 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
             size_t bytes;
         } ups[] = {{z[0], t->kid5.data(), words[0] * 8},  {val[0], t->val5.data(), words[0] * 8},
                    {z[1], t->kid4.data(), words[1] * 8},  {val[1], t->val4.data(), words[1] * 8},
-                   {z[2], t->val3.data(), words[2] * 8},  {pre[0], pre5.data(), words[0] * 4},
-                   {pre[1], pre4.data(), words[1] * 4},   {first[0], t->first4.data(), n5 * 4},
+                   {z[2], t->val3.data(), words[2] * 8},  {first[0], t->first4.data(), n5 * 4},
                    {first[1], t->first3.data(), n4 * 4},  {at_root, root.data(), root.size() * 16},
                    {org[0], o5.data(), n5 * 16}};
         for (auto &u : ups)
             if (u.bytes) WX_CUDA(ctx, cudaMemcpy(base + u.at, u.src, u.bytes, cudaMemcpyHostToDevice));
         const cudaStream_t st = nullptr;
         uint32_t *const ctl = u32(at_ctl);
-        auto *const left = reinterpret_cast<unsigned long long *>(base + at_ctl + 16);
+        auto *const left = reinterpret_cast<unsigned long long *>(base + at_ctl + 32);
         WX_CUDA(ctx, cudaMemsetAsync(ctl, 0, 64, st));
-        if (n3) WX_CUDA(ctx, cudaMemsetAsync((void *)gr->g.leaf, 0, n3 * kN3Slots, st));
         WX_CUDA(ctx, wxk::sdf_child_table(u64(z[0]), u32(pre[0]), u32(first[0]), n5, 15, u32(cidx[0]), st));
         WX_CUDA(ctx, wxk::sdf_child_table(u64(z[1]), u32(pre[1]), u32(first[1]), n4, 12, u32(cidx[1]), st));
         WX_CUDA(ctx, wxk::sdf_child_origins(u32(cidx[0]), i4(org[0]), n5, 5, 7, i4(org[1]), st));
@@ -790,33 +767,32 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
         wxk::SdfWork work{};
         for (int l = 0; l < 3; l++) {
             WX_CUDA(ctx, wxk::sdf_neighbours(5 - l, i4(org[l]), (uint32_t)nodes[l], tree, u32(nb[l]), st));
+            const size_t set = (words[l] + node_words[l]) * 8, real = words[l] * 8;
             if (nodes[l]) {
-                WX_CUDA(ctx, cudaMemsetAsync(base + act[l], 0, nodes[l] * 4, st));
-                WX_CUDA(ctx, cudaMemcpyAsync(base + f[l][0], base + z[l], words[l] * 8, cudaMemcpyDeviceToDevice, st));
-                WX_CUDA(ctx, cudaMemcpyAsync(base + w[l][0], base + z[l], words[l] * 8, cudaMemcpyDeviceToDevice, st));
+                WX_CUDA(ctx, cudaMemsetAsync(base + act[l], 0, (nodes[l] + 1) * 4, st));
+                // The missing neighbour's ones, in z and the W sets.
+                WX_CUDA(ctx, cudaMemset2DAsync(base + z[l] + real, set, 0xFF, set - real, wxk::kSdfWindow + 1, st));
             }
-            WX_CUDA(ctx, wxk::sdf_count_clear(u64(z[l]), words[l], left, st));
-            if (l == 2) {
-                WX_CUDA(ctx, wxk::sdf_count_clear(u64(z[l]), words[l], left + 2, st));
-                WX_CUDA(ctx, cudaMemcpyAsync(left + 1, left + 2, 8, cudaMemcpyDeviceToDevice, st));
-            } else WX_CUDA(ctx, wxk::sdf_pack_internal(u64(z[l]), u64(val[l]), u32(cidx[l]), words[l] * 64, slots[l], st));
-            work.lv[l] = wxk::SdfLevel{u64(z[l]),  l < 2 ? u64(val[l]) : nullptr, {u64(f[l][0]), u64(f[l][1])},
-                                       {u64(w[l][0]), u64(w[l][1])}, u32(nb[l]), u32(act[l]), l < 2 ? slots[l] : nullptr,
-                                       (uint32_t)nodes[l]};
+            WX_CUDA(ctx, wxk::sdf_count_clear(u64(z[l]), words[l], left + l, st));
+            work.lv[l] = wxk::SdfLevel{u64(z[l]), (uint32_t)(set / 8), l < 2 ? u64(val[l]) : nullptr, u32(nb[l]), u32(act[l]),
+                                       l < 2 ? slots[l] : nullptr, (uint32_t)nodes[l]};
         }
+        WX_CUDA(ctx, cudaMemcpyAsync(left + 3, left + 2, 8, cudaMemcpyDeviceToDevice, st));
         work.leaf = const_cast<uint8_t *>(gr->g.leaf);
         work.ctl = ctl;
         work.left = left;
         // Distances below 255 first; the leaf cells then left are the overflow entries.
         struct {
-            uint32_t ctl[4];
-            unsigned long long left[3];  // [2] the inactive leaf cells, as counted at the start
+            uint32_t ctl[8];
+            unsigned long long left[4];  // [3] the inactive leaf cells, as counted at the start
         } h;
-        WX_CUDA(ctx, wxk::sdf_levels(work, 1, 254, ctx->num_sms, ctx->sdf_spins, st));
+        WX_CUDA(ctx, wxk::sdf_levels(work, 1, wxk::kSdfWindow, ctx->num_sms, ctx->sdf_spins, st));
+        WX_CUDA(ctx, wxk::sdf_expand(work, u32(cidx[0]), u32(cidx[1]), st));
+        WX_CUDA(ctx, wxk::sdf_levels(work, wxk::kSdfWindow + 1, 254, ctx->num_sms, ctx->sdf_spins, st));
         WX_CUDA(ctx, wxk::build_top_table(gr->g, st));
         WX_CUDA(ctx, cudaMemcpy(&h, ctl, sizeof h, cudaMemcpyDeviceToHost));
-        if (!h.ctl[2] && h.left[0]) {
-            const uint64_t n_ovf = h.left[1];
+        if (!h.ctl[2] && (h.left[0] | h.left[1] | h.left[2])) {
+            const uint64_t n_ovf = h.left[2];
             if (n_ovf && (rc = alloc_overflow(ctx, gr, n_ovf)) != WX_OK) return rc;
             work.ovf = gr->ovf;
             work.ovf_cap = (uint32_t)n_ovf;
@@ -826,8 +802,8 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
             if (n_ovf && !h.ctl[2] && (rc = sort_overflow(ctx, gr)) != WX_OK) return rc;
         }
         if (h.ctl[2]) return fail(ctx, WX_ERR_TIMEOUT, "wx_grid_build_gpu: the distance steps' barrier wait hit its bound");
-        if (h.left[0]) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build_gpu: distances above 4095");
-        gr->info.active_voxels = n3 * kN3Slots - h.left[2];
+        if (h.left[0] | h.left[1] | h.left[2]) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build_gpu: distances above 4095");
+        gr->info.active_voxels = n3 * kN3Slots - h.left[3];
         guard.g = nullptr;
         *out = gr;
         return WX_OK;

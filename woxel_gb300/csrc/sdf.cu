@@ -27,14 +27,16 @@
 // same time, on bit masks, 64 cells an instruction.
 //
 // k_sdf_levels advances all nodes of all three levels by one k between two
-// barriers of a cooperative grid, in F and W masks that are double-buffered by
-// the parity of k, and writes a cell's distance straight into the grid's pools
-// when it enters W. A container is advanced only when it or one of its
-// 26 neighbours changed in the previous step (act = the last such step). The
-// barrier's wait is bounded; on the bound an error flag ends the kernel.
-// 2000-sphere grid (476,014 leaves, ten or so steps a level): 2.14 ms, where the sweeps in the
-// sweep's order (one CTA a container, a ready queue, 50 barriers a leaf) took 27.4 ms, bound by
-// the chain of containers that wait for one another; the whole build and a 720p frame 34.5 -> 3.85 ms.
+// barriers of a cooperative grid. The first kSdfWindow steps, in which all but a
+// few cells of a level set get their distance, advance every node, keep their W
+// masks, and store nothing else: k_expand_* then turns the masks into pool words,
+// each written once. Later steps alternate between two masks, advance a node only
+// when it or one of its 26 neighbours changed in the step before (act = the last
+// such step), and store a cell's distance when it enters W. The barrier's wait is
+// bounded; on the bound an error flag ends the kernel.
+// 2000-sphere grid (476,014 leaves, 14 steps, the leaves done after 7): 0.90 ms, where the sweeps
+// in the sweep's order (one CTA a container, a ready queue, 50 barriers a leaf) took 27.4 ms, bound
+// by the chain of containers that wait for one another.
 // Distances are small: a cell at distance k lies in a solid cube of containers
 // of side k / D - 1 (every axis-aligned step toward the origin corner is
 // allowed), so k < 2000 for any grid the pools can hold.
@@ -53,9 +55,9 @@ namespace {
 constexpr uint32_t kNone = 0xFFFFFFFFu;   // no node
 constexpr uint32_t kChild = 0x80000000u;
 
-__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
+__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t *p) {
     uint32_t v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
 
@@ -63,9 +65,26 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
 // Structure: child-index tables, derived origins, initial distances.
 // ---------------------------------------------------------------------------
 
+// pre[node * W + w] = the number of child bits in words 0..w-1 of the node; one warp a node of W (a multiple of 32) words.
+__global__ void k_child_prefix(const uint64_t *__restrict__ kid, uint64_t nodes, uint32_t words, uint32_t *__restrict__ pre) {
+    const uint64_t node = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    if (node >= nodes) return;
+    uint32_t sum = 0;
+    for (uint32_t w = lane; w < words; w += 32u) {
+        const uint32_t n = __popcll(kid[node * words + w]);
+        uint32_t upto = n;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(~0u, upto, o);
+            if ((int)lane >= o) upto += v;
+        }
+        pre[node * words + w] = sum + upto - n;
+        sum += __shfl_sync(~0u, upto, 31);
+    }
+}
+
 // cidx[node * S + s] = DFS index of the child in slot s (first[node] + rank of
-// the child bit among the node's child bits), or kNone. pre[node * W + w] is
-// the number of child bits in words 0..w-1 of the node (host prefix).
+// the child bit among the node's child bits), or kNone. pre: k_child_prefix.
 __global__ void k_child_table(const uint64_t *__restrict__ kid, const uint32_t *__restrict__ pre,
                               const uint32_t *__restrict__ first, uint64_t nslots, int slots_log2,
                               uint32_t *__restrict__ cidx) {
@@ -104,7 +123,7 @@ __global__ void k_count_clear(const uint64_t *__restrict__ w, uint64_t n, unsign
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         c += 64u - __popcll(w[i]);
     for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(~0u, c, o);
-    if ((threadIdx.x & 31u) == 0u) atomicAdd(count, c);
+    if ((threadIdx.x & 31u) == 0u && c) atomicAdd(count, c);
 }
 
 // ---------------------------------------------------------------------------
@@ -135,7 +154,7 @@ __device__ __forceinline__ uint32_t find_n5(const wxk::SdfTree &t, int64_t x, in
 }
 
 // nb[c * 27 + k] = index of the container at origin + (dx, dy, dz) * span,
-// k = (dx+1)*9 + (dy+1)*3 + (dz+1); k = 13 is c itself.
+// k = (dx+1)*9 + (dy+1)*3 + (dz+1); k = 13 is c itself; nc where there is none.
 template <int L>
 __global__ void k_sdf_neighbours(const int4 *__restrict__ org, uint32_t nc, wxk::SdfTree t, uint32_t *__restrict__ nb) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -159,215 +178,251 @@ __global__ void k_sdf_neighbours(const int4 *__restrict__ org, uint32_t nc, wxk:
         const uint32_t s4 = ((uint32_t)((x >> 3) & 15) << 8) | ((uint32_t)((y >> 3) & 15) << 4) | (uint32_t)((z >> 3) & 15);
         n = t.c4[((size_t)n << 12) | s4];
     }
-    nb[i] = n;
+    nb[i] = n == kNone ? nc : n;
 }
 
 // ---------------------------------------------------------------------------
 // The levels of k.
 // ---------------------------------------------------------------------------
+using wxk::SdfLevel;
 using wxk::SdfWork;
 
-constexpr uint64_t kZ0 = 0x0101010101010101ull;  // bit z = 0 of every row of an x slice (8 rows of 8 bits)
-constexpr uint64_t kNotZ7 = 0x7F7F7F7F7F7F7F7Full;
+// Cells as 64-bit words of kRows rows of D cells (z); a node is D slices (x) of kSlice words (y).
+template <int L>
+struct Geo {
+    static constexpr int D = 1 << L, kRows = 64 / D, kSlice = D / kRows, kNode = D * kSlice;
+    static constexpr uint64_t kFirst = L == 3 ? 0x0101010101010101ull : L == 4 ? 0x0001000100010001ull : 0x0000000100000001ull;
+    static constexpr uint64_t kNotLast = ~(kFirst << (D - 1));  // all but the last cell of each row
+};
 
-// The cells of an x slice of a leaf within one step of the cells of the slice around it: q[3 * (dy + 1) + dz + 1]
-// is the slice of the same x in the container at (dy, dz). *zd: one step in z only; *below and *above: their rows
-// y - 1 and y + 1.
-__device__ __forceinline__ uint64_t dilate(const uint64_t q[9], uint64_t *below, uint64_t *above) {
-    const uint64_t g = q[4] | ((q[4] & kNotZ7) << 1) | ((q[4] >> 1) & kNotZ7) | ((q[3] >> 7) & kZ0) | ((q[5] & kZ0) << 7);
-    const uint32_t lo = (uint32_t)(q[1] >> 56), hi = (uint32_t)q[7] & 255u;  // row -1, row 8
-    const uint32_t glo = (lo | (lo << 1) | (lo >> 1) | (uint32_t)(q[0] >> 63) | ((uint32_t)(q[2] >> 49) & 128u)) & 255u;
-    const uint32_t ghi = (hi | (hi << 1) | (hi >> 1) | ((uint32_t)(q[6] >> 7) & 1u) | (((uint32_t)q[8] & 1u) << 7)) & 255u;
-    *below = (g << 8) | glo;
-    *above = (g >> 8) | ((uint64_t)ghi << 56);
-    return g;
+// Where the words of a set begin, for neighbours before (or at) and after the node in DFS order: the missing
+// neighbour, n = V.n, comes after every node and has a word block of ones in z and w.
+struct Sets {
+    uint32_t before, after;
+};
+
+// The words around word yq of slice x (x from -1 to D) of node c: q[3 * (dy + 1) + dz + 1] holds the rows just before,
+// at or after it in y (dy), of the node next in z (dz). No branches: all of the 9 index loads, then all 9 words are in
+// flight together.
+template <int L>
+__device__ __forceinline__ void neighbours(const SdfLevel &V, uint32_t c, int x, int yq, uint32_t n[9]) {
+    using G = Geo<L>;
+    const uint32_t *nb = V.nb + (size_t)c * 27u + (x < 0 ? 0 : x >= G::D ? 18 : 9);
+#pragma unroll
+    for (int dy = 0; dy < 3; dy++) {
+        const int y = yq + dy - 1;
+#pragma unroll
+        for (int dz = 0; dz < 3; dz++) n[3 * dy + dz] = nb[(y < 0 ? 0 : y >= G::kSlice ? 6 : 3) + dz];
+    }
+}
+template <int L, bool kFwd>
+__device__ __forceinline__ void around(const SdfLevel &V, Sets f, uint32_t c, int x, int yq, const uint32_t n[9], uint64_t q[9]) {
+    using G = Geo<L>;
+    const uint32_t sx = (uint32_t)(x & (G::D - 1)) * G::kSlice;
+#pragma unroll
+    for (int i = 0; i < 9; i++) {
+        const uint32_t y = (uint32_t)(yq + i / 3 - 1) & (G::kSlice - 1), at = n[i] * G::kNode + sx + y;
+        q[i] = V.sets[at + ((kFwd ? n[i] > c : n[i] >= c) ? f.after : f.before)];
+    }
 }
 
-// Three leaves of a warp, ten lanes each: lane j holds the slice x = j - 1 (-1 and 8 lie in the neighbours).
-// Returns the lane's count of cells that got their distance.
-__device__ __forceinline__ uint32_t leaf_step(const SdfWork &S, uint32_t k, uint32_t task, uint32_t lane) {
-    const uint32_t grp = lane / 10u, j = lane - grp * 10u, c = task * 3u + grp;
-    const wxk::SdfLevel &V = S.lv[2];
-    const bool run = grp < 3u && c < V.n && V.act[c] + 1u >= k;
-    if (!__any_sync(~0u, run)) return 0;
-    const uint64_t *F = V.f[(k - 1u) & 1u], *W = V.w[(k - 1u) & 1u];
-    const uint32_t dx = j == 0u ? 0u : j == 9u ? 2u : 1u, sx = (j - 1u) & 7u;
-    uint64_t f[9], b[9];
-#pragma unroll
-    for (int q = 0; q < 9; q++) {
-        const uint32_t n = run ? V.nb[(size_t)c * 27u + dx * 9u + q] : kNone;
-        f[q] = b[q] = ~0ull;
-        if (n == kNone) continue;
-        const size_t i = (size_t)n * 8u + sx;
-        if (n < c) f[q] = b[q] = F[i];
-        else if (n > c) {
-            f[q] = V.z[i];
-            b[q] = W[i];
-        } else {
-            f[q] = F[i];
-            b[q] = W[i];
-        }
-    }
+// The cells within one step of the words q in y and z; *below and *above: their rows y - 1 and y + 1.
+template <int L>
+__device__ __forceinline__ uint64_t dilate(const uint64_t q[9], uint64_t *below, uint64_t *above) {
+    using G = Geo<L>;
+    constexpr int R = G::D, T = 64 - R;  // bits of a row, shift of the last row
+    const uint64_t g = q[4] | ((q[4] & G::kNotLast) << 1) | ((q[4] >> 1) & G::kNotLast) | ((q[3] >> (R - 1)) & G::kFirst) |
+                       ((q[5] & G::kFirst) << (R - 1));
+    constexpr uint64_t row = ~0ull >> T;
+    const uint64_t lo = q[1] >> T, hi = q[7] & row;
+    const uint64_t glo = lo | ((lo << 1) & row) | (lo >> 1) | (q[0] >> 63) | (((q[2] >> T) & 1u) << (R - 1));
+    const uint64_t ghi = hi | ((hi << 1) & row) | (hi >> 1) | ((q[6] >> (R - 1)) & 1u) | ((q[8] & 1u) << (R - 1));
+    *below = (g << R) | glo;
+    *above = (g >> R) | (ghi << T);
+    return g;
+}
+// Every cell of the rows y - 1, y, y + 1 within a step: what a word receives from the word beside it in x.
+template <int L>
+__device__ __forceinline__ uint64_t dilate_all(const uint64_t q[9]) {
     uint64_t dn, up;
-    uint64_t g = dilate(f, &dn, &up);
-    uint64_t nf = f[4] | dn | ((f[4] & kNotZ7) << 1) | ((f[3] >> 7) & kZ0);
+    const uint64_t g = dilate<L>(q, &dn, &up);
+    return g | dn | up;
+}
+// What a word receives from its own slice: forward the rows before it and the cell before each cell, backward those after.
+template <int L, bool kFwd>
+__device__ __forceinline__ uint64_t own_slice(const uint64_t q[9], uint64_t dn, uint64_t up) {
+    using G = Geo<L>;
+    return kFwd ? q[4] | dn | ((q[4] & G::kNotLast) << 1) | ((q[3] >> (G::D - 1)) & G::kFirst)
+                : q[4] | up | ((q[4] >> 1) & G::kNotLast) | ((q[5] & G::kFirst) << (G::D - 1));
+}
+
+struct Step {
+    Sets f, b;            // where the forward and the backward pass read
+    uint32_t out_f, out_w;  // where F(k) and W(k) are written
+};
+__device__ __forceinline__ uint32_t f_set(uint32_t k) { return k == 0u ? 0u : wxk::kSdfWindow + 1u + (k & 1u); }
+__device__ __forceinline__ uint32_t w_set(uint32_t k) { return k <= wxk::kSdfWindow ? k : wxk::kSdfWindow - (k & 1u); }
+__device__ __forceinline__ Step step_of(const SdfLevel &V, uint32_t k) {
+    const uint32_t f = f_set(k - 1u) * V.stride, w = w_set(k - 1u) * V.stride;
+    return Step{{f, 0u}, {f, w}, f_set(k) * V.stride, w_set(k) * V.stride};
+}
+
+// Three leaves of a warp, ten lanes each: lane j holds the slice x = j - 1 (-1 and 8 lie in the neighbours), one word.
+// Leaves that nothing changed around are left alone. Returns the lane's count of cells that got their distance.
+__device__ __forceinline__ uint32_t leaf_step(const SdfWork &S, uint32_t k, uint32_t first, uint32_t active, uint32_t lane) {
+    const uint32_t grp = lane / 10u, j = lane - grp * 10u;
+    const SdfLevel &V = S.lv[2];
+    const bool run = grp < 3u && ((active >> grp) & 1u);
+    const uint32_t c = run ? first + grp : first;  // lanes without work read with the first leaf
+    const Step st = step_of(V, k);
+    uint64_t f[9], b[9], dn, up;
+    uint32_t n[9];
+    neighbours<3>(V, c, (int)j - 1, 0, n);
+    around<3, true>(V, st.f, c, (int)j - 1, 0, n, f);
+    around<3, false>(V, st.b, c, (int)j - 1, 0, n, b);
+    uint64_t g = dilate<3>(f, &dn, &up);
+    uint64_t nf = own_slice<3, true>(f, dn, up);
     nf |= __shfl_up_sync(~0u, g | dn | up, 1);
-    g = dilate(b, &dn, &up);
-    uint64_t nw = b[4] | nf | up | ((b[4] >> 1) & kNotZ7) | ((b[5] & kZ0) << 7);
+    g = dilate<3>(b, &dn, &up);
+    uint64_t nw = nf | own_slice<3, false>(b, dn, up);
     nw |= __shfl_down_sync(~0u, g | dn | up, 1);
-    const bool own = run && dx == 1u;
-    const size_t i = (size_t)c * 8u + sx;
+    const bool own = run && j >= 1u && j <= 8u;
+    const uint32_t i = c * 8u + ((j - 1u) & 7u);
     if (own) {
-        V.f[k & 1u][i] = nf;
-        V.w[k & 1u][i] = nw;
+        V.sets[st.out_f + i] = nf;
+        V.sets[st.out_w + i] = nw;
     }
     const uint32_t ch = __ballot_sync(~0u, own && (nf != f[4] || nw != b[4]));
-    if (run && (ch & (0x3FFu << (grp * 10u))))
-        for (uint32_t q = j; q < 27u; q += 10u) {
-            const uint32_t n = V.nb[(size_t)c * 27u + q];
-            if (n != kNone) V.act[n] = k;
-        }
     uint64_t add = own ? nw & ~b[4] : 0ull;
     const uint32_t count = __popcll(add);
+    if (k <= wxk::kSdfWindow) return count;
+    if (run && (ch & (0x3FFu << (grp * 10u))))
+        for (uint32_t q = j; q < 27u; q += 10u) V.act[V.nb[(size_t)c * 27u + q]] = k;
     const uint64_t byte = k < 255u ? k : 255u;
-    unsigned long long *out = reinterpret_cast<unsigned long long *>(S.leaf) + i * 8u;  // 64 bytes: rows y of 8 cells
+    unsigned long long *out = reinterpret_cast<unsigned long long *>(S.leaf) + (size_t)i * 8u;  // 64 bytes: rows y of 8 cells
     for (uint32_t y = 0; add; y++, add >>= 8) {
         const uint64_t row = add & 255u;
         if (!row) continue;
         // Bit z of the row into byte z, times the distance; a cell's byte is 0 until it is set here, once.
-        const uint64_t t = (row * kZ0) & 0x8040201008040201ull;
-        atomicOr(out + y, ((((t & kNotZ7) + kNotZ7) | t) >> 7 & kZ0) * byte);
+        constexpr uint64_t kOnes = Geo<3>::kFirst, kLow7 = Geo<3>::kNotLast;
+        const uint64_t t = (row * kOnes) & 0x8040201008040201ull;
+        atomicOr(out + y, ((((t & kLow7) + kLow7) | t) >> 7 & kOnes) * byte);
         if (k >= 255u)
             for (uint32_t m = (uint32_t)row; m; m &= m - 1u) {
                 const uint32_t p = atomicAdd(S.ctl + 3, 1u);
-                if (p < S.ovf_cap) S.ovf[p] = make_uint2((uint32_t)(i * 64u) + y * 8u + __ffs(m) - 1u, k);
+                if (p < S.ovf_cap) S.ovf[p] = make_uint2(i * 64u + y * 8u + (uint32_t)__ffs(m) - 1u, k);
             }
     }
     return count;
 }
 
-template <int L>
-struct RowOf;
-template <>
-struct RowOf<4> {
-    using T = uint16_t;
-};
-template <>
-struct RowOf<5> {
-    using T = uint32_t;
-};
-
-// Row (x, y) of the cells around container c (x, y from -1 to D), as its cells see it: the sets kFwd ? F or Z : W or
-// F by the order of the containers; *zm, *zp: the cells next to the row in z. Missing containers are all ones.
-template <int L, bool kFwd>
-__device__ __forceinline__ uint32_t row_of(const wxk::SdfLevel &V, uint32_t c, uint32_t par, int x, int y, uint32_t *zm,
-                                           uint32_t *zp) {
-    constexpr int D = 1 << L;
-    using T = typename RowOf<L>::T;
-    const int dx = x < 0 ? 0 : x >= D ? 2 : 1, dy = y < 0 ? 0 : y >= D ? 2 : 1;
-    const size_t at = (size_t)((x & (D - 1)) * D + (y & (D - 1)));
-    uint32_t r[3];
-#pragma unroll
-    for (int dz = 0; dz < 3; dz++) {
-        const uint32_t n = V.nb[(size_t)c * 27u + dx * 9 + dy * 3 + dz];
-        r[dz] = (T)~(T)0;
-        if (n == kNone) continue;
-        const uint64_t *src = kFwd ? (n <= c ? V.f[par] : V.z) : (n >= c ? V.w[par] : V.f[par]);
-        r[dz] = reinterpret_cast<const T *>(src)[(size_t)n * (D * D) + at];
-    }
-    *zm = r[0] >> (D - 1);
-    *zp = (r[2] & 1u) << (D - 1);
-    return r[1];
-}
-template <int L, bool kFwd>
-__device__ __forceinline__ uint32_t dilated_row(const wxk::SdfLevel &V, uint32_t c, uint32_t par, int x, int y) {
-    uint32_t zm, zp;
-    const uint32_t r = row_of<L, kFwd>(V, c, par, x, y, &zm, &zp);
-    return r | (r << 1) | (r >> 1) | zm | zp;
-}
-
-// 32 rows (x, y) of an N4 or N5 node, one a lane.
+// 32 words of an N4 or N5 node, one a lane.
 template <int L>
 __device__ __forceinline__ uint32_t node_step(const SdfWork &S, uint32_t k, uint32_t task, uint32_t lane) {
-    constexpr int D = 1 << L;
-    using T = typename RowOf<L>::T;
-    const wxk::SdfLevel &V = S.lv[5 - L];
-    const uint32_t c = task / (D * D / 32), r = (task % (D * D / 32)) * 32u + lane;
-    if (V.act[c] + 1u < k) return 0;
-    const uint32_t par = (k - 1u) & 1u;
-    const int x = (int)(r >> L), y = (int)(r & (D - 1));
-    uint32_t zm, zp;
-    const uint32_t f = row_of<L, true>(V, c, par, x, y, &zm, &zp);
-    uint32_t nf = f | (f << 1) | zm | dilated_row<L, true>(V, c, par, x, y - 1);
-    for (int dy = -1; dy <= 1; dy++) nf |= dilated_row<L, true>(V, c, par, x - 1, y + dy);
-    const uint32_t w = row_of<L, false>(V, c, par, x, y, &zm, &zp);
-    uint32_t nw = w | nf | (w >> 1) | zp | dilated_row<L, false>(V, c, par, x, y + 1);
-    for (int dy = -1; dy <= 1; dy++) nw |= dilated_row<L, false>(V, c, par, x + 1, y + dy);
-    nf = (T)nf;
-    nw = (T)nw;
-    const size_t i = (size_t)c * (D * D) + r;
-    reinterpret_cast<T *>(V.f[k & 1u])[i] = (T)nf;
-    reinterpret_cast<T *>(V.w[k & 1u])[i] = (T)nw;
-    if (__any_sync(~0u, nf != f || nw != w) && lane < 27u) {
-        const uint32_t n = V.nb[(size_t)c * 27u + lane];
-        if (n != kNone) V.act[n] = k;
-    }
-    const uint32_t add = nw & ~w, tile = add & ~(uint32_t)reinterpret_cast<const T *>(V.val)[i];  // active tiles stay 0
-    for (uint32_t m = tile; m; m &= m - 1u) V.slot[i * D + (uint32_t)(__ffs(m) - 1)] = k;
-    return __popc(add);
+    using G = Geo<L>;
+    const SdfLevel &V = S.lv[5 - L];
+    const uint32_t c = task / (G::kNode / 32), r = (task % (G::kNode / 32)) * 32u + lane;
+    if (k > wxk::kSdfWindow + 1u && V.act[c] + 1u < k) return 0;
+    const Step st = step_of(V, k);
+    const int x = (int)(r / G::kSlice), yq = (int)(r % G::kSlice);
+    uint32_t n[9];
+    uint64_t q[9], dn, up;
+    neighbours<L>(V, c, x, yq, n);
+    around<L, true>(V, st.f, c, x, yq, n, q);
+    dilate<L>(q, &dn, &up);
+    const uint64_t f = q[4];
+    uint64_t nf = own_slice<L, true>(q, dn, up);
+    around<L, false>(V, st.b, c, x, yq, n, q);
+    dilate<L>(q, &dn, &up);
+    const uint64_t w = q[4];
+    uint64_t nw = own_slice<L, false>(q, dn, up);
+    neighbours<L>(V, c, x - 1, yq, n);
+    around<L, true>(V, st.f, c, x - 1, yq, n, q);
+    nf |= dilate_all<L>(q);
+    neighbours<L>(V, c, x + 1, yq, n);
+    around<L, false>(V, st.b, c, x + 1, yq, n, q);
+    nw |= nf | dilate_all<L>(q);
+    const uint32_t i = c * G::kNode + r;
+    V.sets[st.out_f + i] = nf;
+    V.sets[st.out_w + i] = nw;
+    const uint64_t add = nw & ~w;
+    if (k <= wxk::kSdfWindow) return __popcll(add);
+    if (__any_sync(~0u, nf != f || nw != w) && lane < 27u) V.act[V.nb[(size_t)c * 27u + lane]] = k;
+    for (uint64_t m = add & ~V.val[i]; m; m &= m - 1u) V.slot[(size_t)i * 64u + (uint32_t)(__ffsll(m) - 1)] = k;  // active tiles stay 0
+    return __popcll(add);
 }
 
 // Steps k0 to k1, or fewer when every cell has its distance. ctl: [0] arrivals at the barrier, [1] its release
-// (2k + (1 when done)), [2] error flag, [3] overflow entries; left: cells without a distance, of all levels and of
-// the leaves. A cooperative launch: the CTAs wait for one another.
-__global__ void __launch_bounds__(256) k_sdf_levels(const __grid_constant__ SdfWork S, uint32_t k0, uint32_t k1,
+// (8k + a bit for each of N5, N4, leaves that is done), [2] error flag, [3] overflow entries, [4..6] last step of
+// N5, N4, leaves; left: cells of N5, N4 and
+// leaves without a distance. A level takes no part once none is left in it. A cooperative launch: the CTAs wait for
+// one another.
+constexpr uint32_t kLeafChunk = 8;  // groups of three leaves a warp takes at a time, looked over with one load
+// Bound by the latency of its gathers. 2000-sphere grid, 14 steps: 0.76 ms with the two k_expand_* another 0.14 ms; as
+// one kernel that stored every distance by an atomic and marked the neighbours of every change from the first step on,
+// 2.1 ms (of a full step's 670 us the marks took 330 and the atomics 190). 6 CTAs an SM at 40 registers: 1.96 ms for
+// the whole build; 2.04 at 4 CTAs (64 registers), 2.14 at 5, 2.47 at 8 (spills).
+__global__ void __launch_bounds__(256, 6) k_sdf_levels(const __grid_constant__ SdfWork S, uint32_t k0, uint32_t k1,
                                                     uint32_t spin_limit) {
-    __shared__ unsigned long long s_new[2];
-    __shared__ uint32_t s_done;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t t5 = S.lv[0].n * 32u, t4 = t5 + S.lv[1].n * 8u, t3 = t4 + (S.lv[2].n + 2u) / 3u;
+    __shared__ uint32_t s_new[3], s_done;
+    const uint32_t lane = threadIdx.x & 31u, warp = blockIdx.x * 8u + (threadIdx.x >> 5), warps = gridDim.x * 8u;
+    const uint32_t n5 = S.lv[0].n * (Geo<5>::kNode / 32), n4 = S.lv[1].n * (Geo<4>::kNode / 32), n3 = S.lv[2].n;
+    if (threadIdx.x == 0u)
+        s_done = S.ctl[2] ? 7u : (S.left[0] == 0ull ? 1u : 0u) | (S.left[1] == 0ull ? 2u : 0u) | (S.left[2] == 0ull ? 4u : 0u);
+    __syncthreads();
     for (uint32_t k = k0; k <= k1; k++) {
-        if (threadIdx.x < 2u) s_new[threadIdx.x] = 0;
+        const uint32_t done = s_done;
+        if (done == 7u) return;
+        if (threadIdx.x < 3u) s_new[threadIdx.x] = 0;
         __syncthreads();
-        uint32_t upper = 0, leaf = 0;
-        for (uint32_t t = blockIdx.x * 8u + (threadIdx.x >> 5); t < t3; t += gridDim.x * 8u) {
-            if (t < t5) upper += node_step<5>(S, k, t, lane);
-            else if (t < t4) upper += node_step<4>(S, k, t - t5, lane);
-            else leaf += leaf_step(S, k, t - t4, lane);
-        }
-        upper = __reduce_add_sync(~0u, upper);
-        leaf = __reduce_add_sync(~0u, leaf);
-        if (lane == 0u && upper + leaf) {
-            atomicAdd(&s_new[0], (unsigned long long)upper + leaf);
-            atomicAdd(&s_new[1], (unsigned long long)leaf);
+        uint32_t got[3] = {0, 0, 0};
+        if (!(done & 1u))
+            for (uint32_t t = warp; t < n5; t += warps) got[0] += node_step<5>(S, k, t, lane);
+        if (!(done & 2u))
+            for (uint32_t t = warp; t < n4; t += warps) got[1] += node_step<4>(S, k, t, lane);
+        if (!(done & 4u))
+            for (uint32_t first = warp * (3u * kLeafChunk); first < n3; first += warps * (3u * kLeafChunk)) {
+                const uint32_t c = first + lane;
+                uint32_t m = __ballot_sync(~0u, lane < 3u * kLeafChunk && c < n3 && (k <= wxk::kSdfWindow + 1u || S.lv[2].act[c] + 1u >= k));
+                for (uint32_t g = first; m; m >>= 3, g += 3u)
+                    if (m & 7u) got[2] += leaf_step(S, k, g, m & 7u, lane);
+            }
+#pragma unroll
+        for (int l = 0; l < 3; l++) {
+            const uint32_t n = __reduce_add_sync(~0u, got[l]);
+            if (lane == 0u && n) atomicAdd(&s_new[l], n);
         }
         __syncthreads();
         if (threadIdx.x == 0u) {
-            if (s_new[0]) atomicAdd(S.left, 0ull - s_new[0]);
-            if (s_new[1]) atomicAdd(S.left + 1, 0ull - s_new[1]);
+            for (int l = 0; l < 3; l++)
+                if (s_new[l]) atomicAdd(S.left + l, 0ull - s_new[l]);
             __threadfence();
             uint32_t v;
             if (atomicAdd(S.ctl, 1u) == gridDim.x * (k - k0 + 1u) - 1u) {
                 __threadfence();
-                v = 2u * k + (atomicAdd(S.left, 0ull) == 0ull ? 1u : 0u);
+                v = 8u * k;
+                for (uint32_t l = 0; l < 3u; l++) {
+                    v |= atomicAdd(S.left + l, 0ull) == 0ull ? 1u << l : 0u;
+                    if (!((done >> l) & 1u)) S.ctl[4u + l] = k;
+                }
                 atomicExch(S.ctl + 1, v);
             } else {
                 for (uint32_t polls = 1;; polls++) {
-                    v = ld_acquire(S.ctl + 1);
-                    if (v >= 2u * k) break;
-                    if (polls >= spin_limit || ld_acquire(S.ctl + 2) != 0u) {  // every CTA then returns
+                    // Relaxed: an acquire would empty the SM's L1 under the CTAs still at work (the fence below acquires).
+                    v = ld_relaxed(S.ctl + 1);
+                    if (v >= 8u * k) break;
+                    if (polls >= spin_limit || ld_relaxed(S.ctl + 2) != 0u) {  // every CTA then returns
                         atomicExch(S.ctl + 2, 1u);
-                        v = 1u;
+                        v = 7u;
                         break;
                     }
                     __nanosleep(256);
                 }
             }
-            s_done = v & 1u;
+            s_done = v & 7u;
             __threadfence();
         }
         __syncthreads();
-        if (s_done) return;
     }
 }
 
@@ -375,13 +430,65 @@ __global__ void __launch_bounds__(256) k_sdf_levels(const __grid_constant__ SdfW
 // Packing.
 // ---------------------------------------------------------------------------
 
-// Slot words of N5/N4: child -> flag | index, active tile -> 0; the other tiles get their distance from k_sdf_levels.
-__global__ void k_pack_internal(const uint64_t *__restrict__ kid, const uint64_t *__restrict__ val,
-                                const uint32_t *__restrict__ cidx, uint64_t nslots, uint32_t *__restrict__ slot) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nslots) return;
-    const bool k = (kid[i >> 6] >> (i & 63)) & 1u, v = (val[i >> 6] >> (i & 63)) & 1u;
-    slot[i] = k && !v ? kChild | cidx[i] : 0u;
+// Leaf bytes after the first kSdfWindow steps, 64 cells a thread: a cell's distance is the number of kept masks
+// W(0)..W(last) that lack it (added up bit-sliced); cells not in W(last) read 0 so far.
+__global__ void __launch_bounds__(256) k_expand_leaves(const __grid_constant__ SdfWork S) {
+    const SdfLevel &V = S.lv[2];
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= V.n * 8u) return;
+    const uint32_t last = min(S.ctl[6], wxk::kSdfWindow);
+    uint64_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, w = 0;
+    for (uint32_t k = 0; k <= last; k++) {
+        w = V.sets[k * V.stride + i];
+        uint64_t x = ~w, t = c0 & x;
+        c0 ^= x;
+        x = c1 & t;
+        c1 ^= t;
+        t = c2 & x;
+        c2 ^= x;
+        c3 ^= t;
+    }
+    c0 &= w;
+    c1 &= w;
+    c2 &= w;
+    c3 &= w;
+    uint4 *out = reinterpret_cast<uint4 *>(S.leaf) + (size_t)i * 4u;
+    // Bit b of a nibble times (1 + 2^7 + 2^14 + 2^21) has its copy at bit 8b.
+    auto four = [&](uint32_t at) {
+        const uint32_t n0 = (uint32_t)(c0 >> at) & 15u, n1 = (uint32_t)(c1 >> at) & 15u, n2 = (uint32_t)(c2 >> at) & 15u,
+                       n3 = (uint32_t)(c3 >> at) & 15u;
+        return ((n0 * 0x00204081u) & 0x01010101u) | ((n1 * 0x00408102u) & 0x02020202u) |
+               ((n2 * 0x00810204u) & 0x04040404u) | ((n3 * 0x01020408u) & 0x08080808u);
+    };
+#pragma unroll
+    for (uint32_t r = 0; r < 4; r++) out[r] = make_uint4(four(16u * r), four(16u * r + 4u), four(16u * r + 8u), four(16u * r + 12u));
+}
+
+// Slot words of N5/N4, four a thread: active tile -> 0, child -> flag | index, else the distance found in the first
+// kSdfWindow steps (0 so far for a later one).
+__global__ void __launch_bounds__(256) k_expand_nodes(const __grid_constant__ SdfWork S, int level,
+                                                      const uint4 *__restrict__ cidx) {
+    const SdfLevel &V = S.lv[level];
+    const uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x;  // grid: exactly a quarter of the level's slots
+    const uint32_t word = (uint32_t)(i >> 4), bit = (uint32_t)(i & 15u) * 4u, last = min(S.ctl[4 + level], wxk::kSdfWindow);
+    const uint32_t kid = (uint32_t)(V.sets[word] >> bit) & 15u, val = (uint32_t)(V.val[word] >> bit) & 15u;
+    uint32_t in = kid, d = 0;  // a byte a slot
+    auto bytes = [](uint32_t nibble) { return (nibble * 0x00204081u) & 0x01010101u; };
+    for (uint32_t k = 1; k <= last; k++) {
+        d += bytes(in ^ 15u);
+        in = (uint32_t)(V.sets[k * V.stride + word] >> bit) & 15u;
+    }
+    d &= bytes(in & ~val) * 255u;
+    uint4 w = make_uint4(d & 255u, (d >> 8) & 255u, (d >> 16) & 255u, d >> 24);
+    const uint32_t child = kid & ~val;
+    if (child) {
+        const uint4 c = cidx[i];
+        if (child & 1u) w.x = kChild | c.x;
+        if (child & 2u) w.y = kChild | c.y;
+        if (child & 4u) w.z = kChild | c.z;
+        if (child & 8u) w.w = kChild | c.w;
+    }
+    reinterpret_cast<uint4 *>(V.slot)[i] = w;
 }
 
 template <class K>
@@ -400,9 +507,10 @@ unsigned grid_for(uint64_t n, int threads) { return (unsigned)((n + threads - 1)
 
 namespace wxk {
 
-cudaError_t sdf_child_table(const uint64_t *kid, const uint32_t *pre, const uint32_t *first, uint64_t nodes,
+cudaError_t sdf_child_table(const uint64_t *kid, uint32_t *pre, const uint32_t *first, uint64_t nodes,
                             int slots_log2, uint32_t *cidx, cudaStream_t st) {
     const uint64_t n = nodes << slots_log2;
+    if (n) k_child_prefix<<<grid_for(nodes * 32, 256), 256, 0, st>>>(kid, nodes, 1u << (slots_log2 - 6), pre);
     if (n) k_child_table<<<grid_for(n, 256), 256, 0, st>>>(kid, pre, first, n, slots_log2, cidx);
     return cudaGetLastError();
 }
@@ -415,7 +523,7 @@ cudaError_t sdf_child_origins(const uint32_t *cidx, const int4 *org, uint64_t no
 }
 
 cudaError_t sdf_count_clear(const uint64_t *w, uint64_t words, unsigned long long *count, cudaStream_t st) {
-    if (words) k_count_clear<<<std::min(grid_for(words, 256), 4096u), 256, 0, st>>>(w, words, count);
+    if (words) k_count_clear<<<std::min(grid_for(words, 256), 1216u), 256, 0, st>>>(w, words, count);
     return cudaGetLastError();
 }
 
@@ -429,9 +537,10 @@ cudaError_t sdf_neighbours(int level, const int4 *org, uint32_t nc, const SdfTre
 }
 
 cudaError_t sdf_levels(const SdfWork &w, uint32_t k0, uint32_t k1, int num_sms, uint32_t spin_limit, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(w.ctl, 0, 3 * sizeof(uint32_t), st);
+    cudaError_t e = cudaMemsetAsync(w.ctl, 0, 2 * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    const uint64_t tasks = (uint64_t)w.lv[0].n * 32 + (uint64_t)w.lv[1].n * 8 + (w.lv[2].n + 2u) / 3u;
+    const uint64_t tasks = (uint64_t)w.lv[0].n * (Geo<5>::kNode / 32) + (uint64_t)w.lv[1].n * (Geo<4>::kNode / 32) +
+                           (w.lv[2].n + 3u * kLeafChunk - 1u) / (3u * kLeafChunk);
     const uint64_t blocks = std::min<uint64_t>((uint64_t)resident_blocks(k_sdf_levels, 256, 0) * num_sms, (tasks + 7) / 8);
     SdfWork work = w;
     void *args[] = {&work, &k0, &k1, &spin_limit};
@@ -439,9 +548,10 @@ cudaError_t sdf_levels(const SdfWork &w, uint32_t k0, uint32_t k1, int num_sms, 
                                        args, 0, st);
 }
 
-cudaError_t sdf_pack_internal(const uint64_t *kid, const uint64_t *val, const uint32_t *cidx, uint64_t nslots,
-                              uint32_t *slot, cudaStream_t st) {
-    if (nslots) k_pack_internal<<<grid_for(nslots, 256), 256, 0, st>>>(kid, val, cidx, nslots, slot);
+cudaError_t sdf_expand(const SdfWork &w, const uint32_t *cidx5, const uint32_t *cidx4, cudaStream_t st) {
+    if (w.lv[0].n) k_expand_nodes<<<w.lv[0].n * (32768u / 1024u), 256, 0, st>>>(w, 0, reinterpret_cast<const uint4 *>(cidx5));
+    if (w.lv[1].n) k_expand_nodes<<<w.lv[1].n * (4096u / 1024u), 256, 0, st>>>(w, 1, reinterpret_cast<const uint4 *>(cidx4));
+    if (w.lv[2].n) k_expand_leaves<<<grid_for((uint64_t)w.lv[2].n * 8u, 256), 256, 0, st>>>(w);
     return cudaGetLastError();
 }
 

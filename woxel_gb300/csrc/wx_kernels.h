@@ -84,30 +84,37 @@ struct SdfTree {
     uint32_t n5;
     const uint32_t *c5, *c4;
 };
-cudaError_t sdf_child_table(const uint64_t *kid, const uint32_t *pre, const uint32_t *first, uint64_t nodes,
+// pre: a word per mask word, filled here.
+cudaError_t sdf_child_table(const uint64_t *kid, uint32_t *pre, const uint32_t *first, uint64_t nodes,
                             int slots_log2, uint32_t *cidx, cudaStream_t st);
 cudaError_t sdf_child_origins(const uint32_t *cidx, const int4 *org, uint64_t nodes, int log2d, int child_span_log2,
                               int4 *org_child, cudaStream_t st);
 cudaError_t sdf_neighbours(int level, const int4 *org, uint32_t nc, const SdfTree &t, uint32_t *nb, cudaStream_t st);
 // *count += the clear bits of `words` mask words.
 cudaError_t sdf_count_clear(const uint64_t *w, uint64_t words, unsigned long long *count, cudaStream_t st);
+// Steps whose W sets are kept until sdf_expand. Level sets are done after about this many.
+constexpr uint32_t kSdfWindow = 8u;
 // One level of the tree in the distance computation (sdf.cu). Masks are those of the grid (bit = cell, D^3 a node).
 struct SdfLevel {
-    const uint64_t *z;       // the cells that start at distance 0: children, active voxels
+    // kSdfWindow + 3 sets of (n + 1) nodes, `stride` words each. 0: z, the cells that start at distance 0 (children,
+    // active voxels), which is F(0) and W(0); 1..kSdfWindow: W(k), then, for larger k, W(k) in the last of them or the
+    // one before by parity; the two after them: F(k) by parity. Node n, the missing neighbour, is all ones in z and
+    // the W sets.
+    uint64_t *sets;
+    uint32_t stride;
     const uint64_t *val;     // N5/N4: active tiles
-    uint64_t *f[2], *w[2];   // forward and final sets, by the parity of k; set 0 starts as z
-    const uint32_t *nb;      // 27 neighbours of each node
-    uint32_t *act;           // last k at which the node or a neighbour changed; starts at 0
+    const uint32_t *nb;      // 27 neighbours of each node (n where there is none)
+    uint32_t *act;           // n + 1 words: last k at which the node or a neighbour changed; starts at 0
     uint32_t *slot;          // N5/N4: slot words
     uint32_t n;              // nodes
 };
 struct SdfWork {
     SdfLevel lv[3];          // N5, N4, leaves
-    uint8_t *leaf;           // leaf bytes, 0 at the start
+    uint8_t *leaf;           // leaf bytes
     uint2 *ovf;              // (cell, distance) of distances >= 255
     uint32_t ovf_cap;
-    uint32_t *ctl;           // 4 words: barrier arrivals and release, error flag, overflow entries
-    unsigned long long *left;  // cells without a distance: of all levels, of the leaves
+    uint32_t *ctl;           // 7 words: barrier arrivals and release, error flag, overflow entries, last steps
+    unsigned long long *left;  // cells of N5, N4 and leaves without a distance
 };
 // Steps k0..k1 (fewer when *left reaches 0). ctl[2] is set when a wait hit its bound.
 // spin_limit: polls (256 ns apart) a CTA makes at the barrier between two steps before it sets
@@ -115,8 +122,8 @@ struct SdfWork {
 constexpr uint32_t kSdfSpinLimit = 1u << 23;  // about 2 s
 constexpr uint32_t kSdfMaxLevel = 4095u;      // no grid reaches it
 cudaError_t sdf_levels(const SdfWork &w, uint32_t k0, uint32_t k1, int num_sms, uint32_t spin_limit, cudaStream_t st);
-cudaError_t sdf_pack_internal(const uint64_t *kid, const uint64_t *val, const uint32_t *cidx, uint64_t nslots,
-                              uint32_t *slot, cudaStream_t st);
+// Slot words and leaf bytes from the W sets of steps 0..kSdfWindow: after sdf_levels(1, kSdfWindow), before larger k.
+cudaError_t sdf_expand(const SdfWork &w, const uint32_t *cidx5, const uint32_t *cidx4, cudaStream_t st);
 
 // Packing of the flattened view (pack.cu): z slabs of an atlas in device memory, as block rows of nodes. The
 // texel of node idx's slot (x, y, z) is at ((idx' / d^2 * D + z) * h + (idx' / d % d * D + y)) * w + idx' % d * D + x
