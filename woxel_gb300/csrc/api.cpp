@@ -1058,8 +1058,9 @@ int wx_render(wx_ctx *ctx, const wx_grid *grid, const wx_state_uniform *state, u
 
 // ---- batched rendering: many frames of several grids in one persistent launch ----
 static int build_jobs(wx_ctx *ctx, const wx_frame *frames, uint32_t n, std::vector<wxk::Job> &jobs,
-                      uint32_t *total_tiles, uint64_t *rays) {
+                      wxk::GridTable &tab, uint32_t *total_tiles, uint64_t *rays) {
     jobs.clear();
+    tab.n = 0;
     uint64_t tiles = 0, r = 0;
     for (uint32_t i = 0; i < n; i++) {
         const wx_frame &f = frames[i];
@@ -1070,9 +1071,10 @@ static int build_jobs(wx_ctx *ctx, const wx_frame *frames, uint32_t n, std::vect
         if (!device_accessible(f.rgba8) || (f.hits && !device_accessible(f.hits)))
             return fail(ctx, WX_ERR_INVALID, "wx_frame: batched outputs must be device memory");
         if ((uint64_t)f.width * f.height >= (1ull << 32)) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_frame: too large");
-        const wxk::Job j = make_job(f.grid, f.state, f.width, f.height, reinterpret_cast<uint32_t *>(f.rgba8), f.hits,
-                                    (uint32_t)tiles, ctx->tuning);
+        wxk::Job j = make_job(f.grid, f.state, f.width, f.height, reinterpret_cast<uint32_t *>(f.rgba8), f.hits,
+                              (uint32_t)tiles, ctx->tuning);
         if (j.tiles == 0) continue;
+        wxk::index_grid(j, tab);
         jobs.push_back(j);
         tiles += j.tiles;
         r += (uint64_t)(f.width & ~7u) * (f.height & ~3u);
@@ -1090,7 +1092,8 @@ int wx_render_batch(wx_ctx *ctx, const wx_frame *frames, uint32_t n, void *strea
         std::vector<wxk::Job> jobs;
         uint32_t total = 0;
         uint64_t rays = 0;
-        int rc = build_jobs(ctx, frames, n, jobs, &total, &rays);
+        wxk::GridTable tab;
+        int rc = build_jobs(ctx, frames, n, jobs, tab, &total, &rays);
         if (rc != WX_OK) return rc;
         if (jobs.empty()) return WX_OK;
         cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -1114,7 +1117,7 @@ int wx_render_batch(wx_ctx *ctx, const wx_frame *frames, uint32_t n, void *strea
         WX_CUDA(ctx, cudaMemcpyAsync(ctx->jobs_dev, ctx->jobs_host, jobs.size() * sizeof(wxk::Job),
                                      cudaMemcpyHostToDevice, st));
         WX_CUDA(ctx, cudaEventRecord(ctx->jobs_done, st));
-        WX_CUDA(ctx, wxk::launch_batched(ctx->jobs_dev, (uint32_t)jobs.size(), total, ctx->take_counter(), ctx->tuning,
+        WX_CUDA(ctx, wxk::launch_batched(ctx->jobs_dev, (uint32_t)jobs.size(), tab, total, ctx->take_counter(), ctx->tuning,
                                          ctx->num_sms, wxk::all_modes(jobs.data(), jobs.size()), st));
         return WX_OK;
     });
@@ -1127,7 +1130,8 @@ int wx_batch_create(wx_ctx *ctx, const wx_frame *frames, uint32_t n, wx_batch **
         std::vector<wxk::Job> jobs;
         uint32_t total = 0;
         uint64_t rays = 0;
-        int rc = build_jobs(ctx, frames, n, jobs, &total, &rays);
+        wxk::GridTable tab;
+        int rc = build_jobs(ctx, frames, n, jobs, tab, &total, &rays);
         if (rc != WX_OK) return rc;
         auto *b = new (std::nothrow) wx_batch();
         if (!b) return fail(ctx, WX_ERR_OOM, "host allocation failed");
@@ -1153,7 +1157,7 @@ int wx_batch_create(wx_ctx *ctx, const wx_frame *frames, uint32_t n, wx_batch **
             cudaStreamDestroy(cs);
             return bail(e, "cudaStreamBeginCapture");
         }
-        cudaError_t le = b->njobs ? wxk::launch_batched(b->jobs_dev, b->njobs, total, b->counter, ctx->tuning,
+        cudaError_t le = b->njobs ? wxk::launch_batched(b->jobs_dev, b->njobs, tab, total, b->counter, ctx->tuning,
                                                         ctx->num_sms, wxk::all_modes(jobs.data(), jobs.size()), cs)
                                   : cudaMemsetAsync(b->counter, 0, sizeof(uint32_t), cs);
         e = cudaStreamEndCapture(cs, &b->graph);

@@ -36,7 +36,7 @@ using wxk::Job;
 // alternately the rows above and below it (a permutation of the rows).
 __device__ __forceinline__ bool tile_pixel(const Job &J, uint32_t tl, uint32_t lane, uint32_t &gx, uint32_t &gy) {
     uint32_t row = tl / J.tiles_x;
-    if (J.order) {
+    if (J.order & 1u) {
         const uint32_t mid = (J.tiles / J.tiles_x) >> 1;
         row = (row & 1u) ? mid - ((row + 1u) >> 1) : mid + (row >> 1);
     }
@@ -48,7 +48,7 @@ __device__ __forceinline__ bool tile_pixel(const Job &J, uint32_t tl, uint32_t l
 constexpr int kBase = 1, kGlossy = 2, kSurface = 4, kAllModes = 7;
 
 template <int kModes, bool kCompact = false>
-__device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t lane, bool wait_prev) {
+__device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uint32_t tl, uint32_t lane, bool wait_prev) {
     uint32_t gx, gy;
     // The warp's lanes leave each march at different iterations. Without the
     // explicit reconvergence points below they go on in small groups, each
@@ -62,7 +62,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
     const uint32_t pix = gy * J.width + gx;
     if ((kModes & kGlossy) && (kModes == kGlossy || s.render_mode[0] == 4u)) {
         // The hit record is stored at the first hit, so that it is not live across the later rays.
-        const F3 c = glossy_colour(J.g, s, eye, dir, act, [&](const March &hit) {
+        const F3 c = glossy_colour(G, s, eye, dir, act, [&](const March &hit) {
             if (!J.hits) return;
             if (wait_prev) asm volatile("griddepcontrol.wait;" ::: "memory");
             if (wx_in_range(pix, (uint64_t)J.width * J.height))
@@ -73,7 +73,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
         if (wx_in_range(pix, (uint64_t)J.width * J.height)) J.rgba[pix] = pack_rgba(c);
         return;
     }
-    const March hit = hdda(J.g, eye, dir);
+    const March hit = hdda(G, eye, dir);
     __syncwarp(act);
     F3 c;
     uint32_t shadow = 0, reserved = 0;
@@ -83,7 +83,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
             float ts;
             uint32_t ks;
             F3 N;
-            if (surf_search(J.g, eye, dir, dot3(hit.p - eye, dir), &ts, &ks, &N)) {
+            if (surf_search(G, eye, dir, dot3(hit.p - eye, dir), &ts, &ks, &N)) {
                 c = surface_colour(s, N);
                 shadow = 1u | (ks << 8);
                 reserved = __float_as_uint(ts);
@@ -112,7 +112,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
         const uint32_t node = hit.node;
         __syncwarp(act);  // shadow rays of the warp start together
         if (need) {
-            const March sh = hdda(J.g, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
+            const March sh = hdda(G, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
             shadow = 1u | (sh.state << 1) | (sh.i << 8);
             if (sh.state == 0u) cpk = pack_rgba(ambient_colour());  // shadowed is I_a
         }
@@ -128,7 +128,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
         c = primary_colour(s, hit, dir, &need, &shadowed, &src);
         __syncwarp(act);  // shadow rays of the warp start together
         if (need) {
-            const March sh = hdda(J.g, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
+            const March sh = hdda(G, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
             shadow = 1u | (sh.state << 1) | (sh.i << 8);
             if (sh.state == 0u) c = shadowed;
         }
@@ -152,8 +152,9 @@ __device__ __forceinline__ void render_pixel(const Job &J, uint32_t tl, uint32_t
 // 2000 spheres at 1080p take 3.27 ms at 32 registers, 3.47 at 40 and 3.67 at 47 (2 noise frames at
 // 4K: 2.20, 2.23 and 2.29 ms). The glossy kernel takes 0.38 ms for a 720p frame at 40 and 48
 // registers, 0.39 at 32 and 0.42 at 64; a zero-crossing 1080p frame 0.54 ms at 32, 0.58 at 40 and 0.59
-// at 48. The persistent kernels hold the job's pointers in registers and stay at 48
-// (5 blocks, 40 warps): 48 mixed frames take 13.0 ms, 14.2 at 40 registers and 13.4 at 55.
+// at 48. The persistent kernels keep 48 (5 blocks, 40 warps): their warps live on, so that a finished
+// block frees nothing early, and 48 mixed frames take 12.7 ms, 13.5 at 40 registers, 13.3 at 32, 12.9 at 64.
+// (One warp per tile over the job table instead of the queue: 13.9 ms at 32 registers, 13.5 at 48.)
 #define WX_RAY_BOUNDS __launch_bounds__(256, 5)
 #define WX_PIXEL_BOUNDS __launch_bounds__(256, kModes == kGlossy ? 6 : 8)
 
@@ -172,7 +173,7 @@ __global__ void WX_PIXEL_BOUNDS k_pixel(const __grid_constant__ Job job, uint32_
     asm volatile("griddepcontrol.launch_dependents;");
     const uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (tile >= ntiles) return;
-    render_pixel<kModes>(job, tile, threadIdx.x & 31u, disjoint == 0u);
+    render_pixel<kModes>(job, job.g, tile, threadIdx.x & 31u, disjoint == 0u);
 }
 
 // ---------------------------------------------------------------------------
@@ -393,14 +394,20 @@ __device__ __forceinline__ uint32_t find_job(const Job *__restrict__ jobs, uint3
     return lo;
 }
 
+// A job's grid comes from the launch's table of distinct grids, which is a kernel parameter: its pools' addresses
+// are then constant-bank loads, as in k_pixel, instead of registers held through the march (48 mixed frames
+// 13.2 -> 12.7 ms, 60 small frames 1.04 -> 0.98 ms). Launches over more than kTableGrids grids read the job's copy.
+//
 // Persistent warps drawing whole tiles from a global queue (one atomic per
 // 32 rays). Tiles are numbered job by job; a warp's successive tiles increase,
 // so its job search starts at the previous job.
 // Batched launches may carry a cancel table (the server's): a job whose
 // cancel_id has been written to cancel[cancel_slot] (by the host, while the
 // launch runs) has its remaining tiles skipped, which `skipped` counts.
-template <bool kBatched, int kModes>
+enum Batch { kOneJob, kJobGrid, kTableGrid };  // one frame; jobs with their own grids; jobs that index the grid table
+template <Batch kBatch, int kModes>
 __global__ void WX_RAY_BOUNDS k_persistent(const Job *__restrict__ jobs, uint32_t njobs, const __grid_constant__ Job job0,
+                             const __grid_constant__ wxk::GridTable tab,
                              uint32_t total_tiles, uint32_t *__restrict__ ctr, const uint32_t *cancel,
                              uint32_t *skipped) {
     const uint32_t lane = threadIdx.x & 31u;
@@ -410,7 +417,7 @@ __global__ void WX_RAY_BOUNDS k_persistent(const Job *__restrict__ jobs, uint32_
         if (lane == 0) t = atomicAdd(ctr, 1u);
         t = __shfl_sync(~0u, t, 0);
         if (t >= total_tiles) break;
-        if (kBatched) {
+        if (kBatch != kOneJob) {
             cur_job = find_job(jobs, njobs, t, cur_job);
             const Job &J = jobs[cur_job];
             if (cancel) {
@@ -424,9 +431,9 @@ __global__ void WX_RAY_BOUNDS k_persistent(const Job *__restrict__ jobs, uint32_
                     continue;
                 }
             }
-            render_pixel<kModes, true>(J, t - J.tile_begin + J.tile_off, lane, true);
+            render_pixel<kModes, true>(J, kBatch == kTableGrid ? tab.g[J.order >> 8] : J.g, t - J.tile_begin + J.tile_off, lane, true);
         } else {
-            render_pixel<kModes, true>(job0, t, lane, true);
+            render_pixel<kModes, true>(job0, job0.g, t, lane, true);
         }
     }
 }
@@ -499,7 +506,7 @@ cudaError_t build_top_table(const DevGrid &g, cudaStream_t st) {
 int max_blocks_per_sm(int kernel, bool batched, int warps_per_block) {
     const int threads = 32 * warps_per_block;
     if (kernel == 1) return blocks_for(k_pixel<kBase>, threads);
-    return batched ? blocks_for(k_persistent<true, kBase>, threads) : blocks_for(k_persistent<false, kBase>, threads);
+    return batched ? blocks_for(k_persistent<kTableGrid, kBase>, threads) : blocks_for(k_persistent<kOneJob, kBase>, threads);
 }
 
 cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, cudaStream_t st) {
@@ -543,27 +550,36 @@ cudaError_t launch_persistent(const Job &job, uint32_t *ctr, const Tuning &t, in
     if (e != cudaSuccess) return e;
     const int blocks = grid_blocks(t, false, num_sms, job.tiles);
     if (all_modes(job.s))
-        k_persistent<false, kAllModes><<<blocks, 32 * t.warps_per_block, 0, st>>>(nullptr, 1, job, job.tiles, ctr, nullptr,
+        k_persistent<kOneJob, kAllModes><<<blocks, 32 * t.warps_per_block, 0, st>>>(nullptr, 1, job, wxk::GridTable{}, job.tiles, ctr, nullptr,
                                                                             nullptr);
     else
-        k_persistent<false, kBase><<<blocks, 32 * t.warps_per_block, 0, st>>>(nullptr, 1, job, job.tiles, ctr, nullptr,
+        k_persistent<kOneJob, kBase><<<blocks, 32 * t.warps_per_block, 0, st>>>(nullptr, 1, job, wxk::GridTable{}, job.tiles, ctr, nullptr,
                                                                              nullptr);
     return cudaGetLastError();
 }
 
-cudaError_t launch_batched(const Job *jobs_dev, uint32_t njobs, uint32_t total_tiles, uint32_t *ctr,
+void index_grid(Job &job, GridTable &tab) {
+    uint32_t i = 0;
+    while (i < tab.n && i < kTableGrids && memcmp(&tab.g[i], &job.g, sizeof(DevGrid)) != 0) i++;
+    if (i == tab.n && i < kTableGrids) tab.g[tab.n++] = job.g;
+    else if (i == kTableGrids) tab.n = kTableGrids + 1;
+    job.order = (job.order & 1u) | (i << 8);
+}
+
+cudaError_t launch_batched(const Job *jobs_dev, uint32_t njobs, const GridTable &tab, uint32_t total_tiles, uint32_t *ctr,
                            const Tuning &t, int num_sms, bool all, cudaStream_t st, const uint32_t *cancel,
                            uint32_t *skipped) {
     cudaError_t e = cudaMemsetAsync(ctr, 0, sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
-    Job dummy{};
-    const int blocks = grid_blocks(t, true, num_sms, total_tiles);
-    if (all)
-        k_persistent<true, kAllModes><<<blocks, 32 * t.warps_per_block, 0, st>>>(jobs_dev, njobs, dummy, total_tiles, ctr,
-                                                                           cancel, skipped);
-    else
-        k_persistent<true, kBase><<<blocks, 32 * t.warps_per_block, 0, st>>>(jobs_dev, njobs, dummy, total_tiles, ctr,
-                                                                            cancel, skipped);
+    const Job dummy{};
+    const int blocks = grid_blocks(t, true, num_sms, total_tiles), threads = 32 * t.warps_per_block;
+    if (tab.n > kTableGrids) {
+        if (all) k_persistent<kJobGrid, kAllModes><<<blocks, threads, 0, st>>>(jobs_dev, njobs, dummy, tab, total_tiles, ctr, cancel, skipped);
+        else k_persistent<kJobGrid, kBase><<<blocks, threads, 0, st>>>(jobs_dev, njobs, dummy, tab, total_tiles, ctr, cancel, skipped);
+    } else {
+        if (all) k_persistent<kTableGrid, kAllModes><<<blocks, threads, 0, st>>>(jobs_dev, njobs, dummy, tab, total_tiles, ctr, cancel, skipped);
+        else k_persistent<kTableGrid, kBase><<<blocks, threads, 0, st>>>(jobs_dev, njobs, dummy, tab, total_tiles, ctr, cancel, skipped);
+    }
     return cudaGetLastError();
 }
 
@@ -727,10 +743,13 @@ int noalloc_render(int device, const wx_frame *frames, uint32_t n, cudaStream_t 
     uint32_t njobs = 0;
     uint64_t tiles = 0;
     bool all = false;
+    wxk::GridTable tab;
+    tab.n = 0;
     for (uint32_t i = 0; i < n; i++) {
         Job &j = chunk.jobs[0];
         if ((rc = noalloc_job(frames[i], device, tiles, j)) != WX_OK) return rc;
         if (j.tiles == 0) continue;
+        wxk::index_grid(j, tab);
         tiles += j.tiles;
         all = all || wxk::all_modes(j.s);
         njobs++;
@@ -744,6 +763,7 @@ int noalloc_render(int device, const wx_frame *frames, uint32_t n, cudaStream_t 
         Job &j = chunk.jobs[chunk.count];
         noalloc_job(frames[i], device, tiles, j);
         if (j.tiles == 0) continue;
+        wxk::index_grid(j, tab);  // the place found in pass 1
         tiles += j.tiles;
         if (++chunk.count == kTableChunk || chunk.first + chunk.count == njobs) {
             k_noalloc_table<<<1, 256, 0, st>>>(chunk);
@@ -756,7 +776,7 @@ int noalloc_render(int device, const wx_frame *frames, uint32_t n, cudaStream_t 
     Job *jobs_dev = reinterpret_cast<Job *>(d->scratch + kNoallocJobsOffset);
     uint32_t *counter = reinterpret_cast<uint32_t *>(d->scratch);
     wxk::Tuning t;  // defaults; launch_batched clears the counter (it keeps the last call's value otherwise)
-    const cudaError_t e = wxk::launch_batched(jobs_dev, njobs, (uint32_t)tiles, counter, t, d->num_sms, all, st);
+    const cudaError_t e = wxk::launch_batched(jobs_dev, njobs, tab, (uint32_t)tiles, counter, t, d->num_sms, all, st);
     if (e != cudaSuccess) return noalloc_fail(WX_ERR_CUDA, "wx_render_batch_noalloc: launch failed");
     return WX_OK;
 }

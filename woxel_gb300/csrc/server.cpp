@@ -207,6 +207,8 @@ struct wx_server {
     bool launch(Slot &s) {
         const bool fifo = cfg.flags & WX_SERVE_FIFO;
         uint32_t budget = fifo ? UINT32_MAX : cfg.slice_tiles, tiles = 0, n = 0;
+        wxk::GridTable tab;
+        tab.n = 0;
         for (Req *q : active) {
             if (q->next < q->tiles && q->status != WX_OK) {  // failed or cancelled: give up its remaining tiles
                 const uint32_t rest = q->tiles - q->next;
@@ -234,6 +236,7 @@ struct wx_server {
             j.s = q->r.state;
             j.cancel_slot = (uint32_t)(q->ticket % kCancelSlots);
             j.cancel_id = (uint32_t)q->ticket;
+            wxk::index_grid(j, tab);
             s.parts.emplace_back(q, take);
             q->next += take;
             tiles += take;
@@ -246,7 +249,7 @@ struct wx_server {
         cudaError_t e = cudaMemcpyAsync(s.jobs_dev, s.jobs_host, n * sizeof(wxk::Job), cudaMemcpyHostToDevice, s.stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(s.counter, 0, 2 * sizeof(uint32_t), s.stream);
         if (e == cudaSuccess)
-            e = wxk::launch_batched(s.jobs_dev, n, tiles, s.counter, t, num_sms, wxk::all_modes(s.jobs_host, n),
+            e = wxk::launch_batched(s.jobs_dev, n, tab, tiles, s.counter, t, num_sms, wxk::all_modes(s.jobs_host, n),
                                     s.stream, cancel_dev, s.counter + 1);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(s.skipped_host, s.counter + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s.stream);

@@ -33,7 +33,8 @@ struct Job {
     DevGrid g;
     uint32_t width, height;
     uint16_t tile_w, tile_h;       // pixel tile of one warp (tile_w * tile_h = 32)
-    uint32_t order;                // tile rows: 0 top to bottom, 1 middle row first, then outwards
+    uint32_t order;                // bit 0, tile rows: 0 top to bottom, 1 middle row first, then outwards;
+                                   // from bit 8: the grid's place in the launch's GridTable
     uint32_t tiles_x, tiles;       // tiles per row / per frame over the dispatched region
     uint32_t tile_begin;           // first global (queue) tile id of this job
     uint32_t tile_off;             // first frame tile of this job (a job may cover part of a frame)
@@ -43,6 +44,14 @@ struct Job {
     // Cancellation (batched launches given a cancel table): the job's tiles are
     // skipped once cancel[cancel_slot] == cancel_id (nonzero). 0 = never.
     uint32_t cancel_slot, cancel_id;
+};
+
+// The distinct grids of a batched launch, a kernel parameter; n = 0 when there are more than kTableGrids (the jobs'
+// own copies are then used).
+constexpr uint32_t kTableGrids = 64;
+struct GridTable {
+    DevGrid g[kTableGrids];
+    uint32_t n;
 };
 
 struct Tuning {
@@ -65,9 +74,12 @@ cudaError_t launch_persistent(const Job &job, uint32_t *ctr, const Tuning &t, in
 // all: some job renders mode 4 or 5 (the kernels compiled for every mode).
 // cancel (may be NULL): the table the jobs' cancel_slot index; skipped (may be
 // NULL) counts the tiles skipped for a cancelled job (the caller clears it).
-cudaError_t launch_batched(const Job *jobs_dev, uint32_t njobs, uint32_t total_tiles, uint32_t *ctr,
+// tab: index_grid of every job, which must be done before the jobs are copied to jobs_dev.
+cudaError_t launch_batched(const Job *jobs_dev, uint32_t njobs, const GridTable &tab, uint32_t total_tiles, uint32_t *ctr,
                            const Tuning &t, int num_sms, bool all, cudaStream_t st,
                            const uint32_t *cancel = nullptr, uint32_t *skipped = nullptr);
+// Enters the job's grid into the table (unless it has overflowed: n = kTableGrids + 1) and its place into job.order.
+void index_grid(Job &job, GridTable &tab);
 // Modes 4 (glossy) and 5 (zero crossing) need the kernels compiled for every mode.
 bool all_modes(const wx_state_uniform &s);
 bool all_modes(const Job *jobs, size_t n);
