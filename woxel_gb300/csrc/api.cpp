@@ -131,8 +131,8 @@ std::vector<PixelOutputs> g_pixel_outputs;
 // cudaStreamPerThread is one handle for a different stream in every host thread,
 // so no record can name its predecessor: frames on it always wait. NULL and
 // cudaStreamLegacy name the same stream.
-cudaError_t launch_pixel_tracked(const wxk::Job &job, const wxk::Tuning &t, PixelOutputs cur) {
-    if (cur.stream == cudaStreamPerThread) return wxk::launch_pixel(job, t, false, cur.stream);
+cudaError_t launch_pixel_tracked(const wxk::Job &job, const wxk::Tuning &t, int num_sms, PixelOutputs cur) {
+    if (cur.stream == cudaStreamPerThread) return wxk::launch_pixel(job, t, false, num_sms, cur.stream);
     if (cur.stream == cudaStreamLegacy) cur.stream = nullptr;
     auto meet = [](uintptr_t a0, uintptr_t a1, uintptr_t b0, uintptr_t b1) {
         return a0 < a1 && b0 < b1 && a0 < b1 && b0 < a1;
@@ -151,7 +151,7 @@ cudaError_t launch_pixel_tracked(const wxk::Job &job, const wxk::Tuning &t, Pixe
     } else if (v.size() >= kPixelStreams) {
         v.erase(v.begin());
     }
-    const cudaError_t e = wxk::launch_pixel(job, t, disjoint, cur.stream);
+    const cudaError_t e = wxk::launch_pixel(job, t, disjoint, num_sms, cur.stream);
     if (e == cudaSuccess) v.push_back(cur);  // after a failed launch the stream's last kernel is unknown
     return e;
 }
@@ -1039,7 +1039,7 @@ int wx_render(wx_ctx *ctx, const wx_grid *grid, const wx_state_uniform *state, u
                 cur.lo[1] = reinterpret_cast<uintptr_t>(out_hits);
                 cur.hi[1] = cur.lo[1] + npix * sizeof(wx_hit);
             }
-            const cudaError_t e = launch_pixel_tracked(job, ctx->tuning, cur);
+            const cudaError_t e = launch_pixel_tracked(job, ctx->tuning, ctx->num_sms, cur);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "wxk::launch_pixel");
         } else {
             WX_CUDA(ctx, wxk::launch_persistent(job, ctx->take_counter(), ctx->tuning, ctx->num_sms, st));

@@ -48,13 +48,14 @@ __device__ __forceinline__ bool tile_pixel(const Job &J, uint32_t tl, uint32_t l
 constexpr int kBase = 1, kGlossy = 2, kSurface = 4, kAllModes = 7;
 
 template <int kModes, bool kCompact = false>
-__device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uint32_t tl, uint32_t lane, bool wait_prev) {
+__device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uint32_t tl, uint32_t lane, bool wait_prev,
+                                             uint32_t lanes = ~0u) {  // lanes: the warp's lanes that are here
     uint32_t gx, gy;
     // The warp's lanes leave each march at different iterations. Without the
     // explicit reconvergence points below they go on in small groups, each
     // running the shading once and starting its own shadow march.
     const bool valid = tile_pixel(J, tl, lane, gx, gy);
-    const uint32_t act = __ballot_sync(~0u, valid);
+    const uint32_t act = __ballot_sync(lanes, valid);
     if (!valid) return;
     const wx_state_uniform &s = J.s;
     const F3 dir = primary_dir(s, gx, gy);
@@ -167,13 +168,17 @@ __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uin
 // host when this frame's outputs do not overlap that frame's) lets every block
 // write without waiting and retire as soon as its tiles are done, so the
 // previous frame's last blocks do not hold finished blocks on the SMs.
+//
+// split: 2^split warps share a tile, each with the first 32 >> split of its lanes. A small frame leaves the chip idle
+// and takes as long as its slowest warp; with fewer rays a warp, an iteration resolves fewer levels in turn and no ray
+// waits for 31 others. See pixel_split.
 template <int kModes>
-__global__ void WX_PIXEL_BOUNDS k_pixel(const __grid_constant__ Job job, uint32_t ntiles, uint32_t disjoint) {
+__global__ void WX_PIXEL_BOUNDS k_pixel(const __grid_constant__ Job job, uint32_t ntiles, uint32_t disjoint, uint32_t split) {
     if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
-    const uint32_t tile = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (tile >= ntiles) return;
-    render_pixel<kModes>(job, job.g, tile, threadIdx.x & 31u, disjoint == 0u);
+    const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u, n = 32u >> split;
+    if ((warp >> split) >= ntiles || lane >= n) return;
+    render_pixel<kModes>(job, job.g, warp >> split, (warp & ((1u << split) - 1u)) * n + lane, disjoint == 0u, ~0u >> (32u - n));
 }
 
 // ---------------------------------------------------------------------------
@@ -509,13 +514,22 @@ int max_blocks_per_sm(int kernel, bool batched, int warps_per_block) {
     return batched ? blocks_for(k_persistent<kTableGrid, kBase>, threads) : blocks_for(k_persistent<kOneJob, kBase>, threads);
 }
 
-cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, cudaStream_t st) {
-    const uint32_t wpb = (uint32_t)t.warps_per_block;
+// Warps a tile: as many, up to 8, as keep the frame's warps within 28 an SM (of 64). Mode 3 over 500 spheres and over
+// one, queued frames, us at 1, 2, 4 and 8 warps a tile: 192 tiles 94, 63, 56, 51 and 44, 30, 27, 25; 600 tiles 74, 65,
+// 62, 62 and 34, 30, 27, 28; 2048 tiles 82, 74, 77, 101 and 33, 32, 37, 60; 3750 tiles 85, 84, 96, 152 and 34, 36, 53, 99.
+static uint32_t pixel_split(uint32_t tiles, int num_sms) {
+    uint32_t s = 0;
+    while (s < 3u && ((uint64_t)tiles << (s + 1u)) <= (uint64_t)num_sms * 28u) s++;
+    return s;
+}
+
+cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, int num_sms, cudaStream_t st) {
+    const uint32_t wpb = (uint32_t)t.warps_per_block, split = pixel_split(job.tiles, num_sms);
     // Programmatic dependent launch: back-to-back frames on one stream overlap
     // the previous frame's last blocks with this frame's march (the kernel's
     // stores wait for the previous kernel; see render_pixel).
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((job.tiles + wpb - 1) / wpb);
+    cfg.gridDim = dim3((unsigned)((((uint64_t)job.tiles << split) + wpb - 1) / wpb));
     cfg.blockDim = dim3(32 * wpb);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -524,8 +538,8 @@ cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, cudaStr
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const uint32_t dj = disjoint ? 1u : 0u;
-    if (job.s.render_mode[0] == 4u) return cudaLaunchKernelEx(&cfg, k_pixel<kGlossy>, job, job.tiles, dj);
-    if (job.s.render_mode[0] == 5u) return cudaLaunchKernelEx(&cfg, k_pixel<kSurface>, job, job.tiles, dj);
+    if (job.s.render_mode[0] == 4u) return cudaLaunchKernelEx(&cfg, k_pixel<kGlossy>, job, job.tiles, dj, split);
+    if (job.s.render_mode[0] == 5u) return cudaLaunchKernelEx(&cfg, k_pixel<kSurface>, job, job.tiles, dj, split);
     if (t.rays > 1) {  // k_wave: t.rays tiles per warp, lanes refill
         const uint32_t per_block = wpb * (uint32_t)t.rays;
         cfg.gridDim = dim3((job.tiles + per_block - 1) / per_block);
@@ -534,7 +548,7 @@ cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, cudaStr
         if (t.rays == 4) return cudaLaunchKernelEx(&cfg, k_wave<4>, job, job.tiles, dj);
         return cudaLaunchKernelEx(&cfg, k_wave<8>, job, job.tiles, dj);
     }
-    return cudaLaunchKernelEx(&cfg, k_pixel<kBase>, job, job.tiles, dj);
+    return cudaLaunchKernelEx(&cfg, k_pixel<kBase>, job, job.tiles, dj, split);
 }
 
 static int grid_blocks(const Tuning &t, bool batched, int num_sms, uint32_t total_tiles) {

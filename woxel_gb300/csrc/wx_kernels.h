@@ -69,7 +69,7 @@ cudaError_t build_top_table(const DevGrid &g, cudaStream_t st);
 int max_blocks_per_sm(int kernel, bool batched, int warps_per_block);
 // disjoint: the job's outputs do not overlap those of the previous kernel on st,
 // a k_pixel launch (see k_pixel); false is always safe.
-cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, cudaStream_t st);
+cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, int num_sms, cudaStream_t st);
 cudaError_t launch_persistent(const Job &job, uint32_t *ctr, const Tuning &t, int num_sms, cudaStream_t st);
 // all: some job renders mode 4 or 5 (the kernels compiled for every mode).
 // cancel (may be NULL): the table the jobs' cancel_slot index; skipped (may be
