@@ -47,7 +47,7 @@ __device__ __forceinline__ bool tile_pixel(const Job &J, uint32_t tl, uint32_t l
 
 constexpr int kBase = 1, kGlossy = 2, kSurface = 4, kAllModes = 7;
 
-template <int kModes, bool kCompact = false>
+template <int kModes>
 __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uint32_t tl, uint32_t lane, bool wait_prev,
                                              uint32_t lanes = ~0u) {  // lanes: the warp's lanes that are here
     uint32_t gx, gy;
@@ -97,12 +97,11 @@ __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uin
             F3 shadowed, src;
             c = primary_colour(s, hit, dir, &need, &shadowed, &src);  // states 1, 2: mode 3's colours
         }
-    } else if (kCompact) {  // modes 0-3 in the persistent kernels
+    } else {  // modes 0-3: every valid lane of the warp comes here (the __syncwarp below needs them all)
         // Everything the stores need is reduced to a few words before the shadow
         // march (the packed colour, t, the info word), so that the direction and
-        // both candidate colours are not live across it: the persistent kernels
-        // then spill 32 bytes instead of 92 and the mixed batch runs at 4.80
-        // instead of 4.58 Grays/s (k_pixel, with fewer registers, gains nothing).
+        // both candidate colours are not live across it: 8 frames of 2000 spheres at
+        // 1080p 3.29 -> 3.25 ms, 2 noise frames at 4K 2.23 -> 2.18 ms.
         bool need;
         F3 shadowed, src;
         const F3 cc = primary_colour(s, hit, dir, &need, &shadowed, &src);
@@ -123,16 +122,6 @@ __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uin
         J.rgba[pix] = cpk;
         if (J.hits) store_hit(J.hits + pix, hp, t, node, info, shadow, 0u);
         return;
-    } else {  // modes 0-3: every valid lane of the warp comes here (the __syncwarp below needs them all)
-        bool need;
-        F3 shadowed, src;
-        c = primary_colour(s, hit, dir, &need, &shadowed, &src);
-        __syncwarp(act);  // shadow rays of the warp start together
-        if (need) {
-            const March sh = hdda(G, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
-            shadow = 1u | (sh.state << 1) | (sh.i << 8);
-            if (sh.state == 0u) c = shadowed;
-        }
     }
     __syncwarp(act);
     // A programmatically dependent launch (k_pixel) may run its march while the
@@ -149,9 +138,9 @@ __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uin
 
 // Blocks of at most 256 threads. k_pixel in modes 0-3: 8 resident, 32 registers a thread, all 64
 // warp slots of an SM. Its march waits on dependent loads and leaves a third of its lanes idle, so
-// resident warps pay more than the five reloads an iteration that 32 registers cost: 8 frames of
-// 2000 spheres at 1080p take 3.27 ms at 32 registers, 3.47 at 40 and 3.67 at 47 (2 noise frames at
-// 4K: 2.20, 2.23 and 2.29 ms). The glossy kernel takes 0.38 ms for a 720p frame at 40 and 48
+// resident warps pay more than the three reloads an iteration that 32 registers cost: 8 frames of
+// 2000 spheres at 1080p take 3.25 ms at 32 registers, 3.47 at 40 and 3.67 at 47 (2 noise frames at
+// 4K: 2.18, 2.23 and 2.29 ms). The glossy kernel takes 0.38 ms for a 720p frame at 40 and 48
 // registers, 0.39 at 32 and 0.42 at 64; a zero-crossing 1080p frame 0.54 ms at 32, 0.58 at 40 and 0.59
 // at 48. The persistent kernels keep 48 (5 blocks, 40 warps): their warps live on, so that a finished
 // block frees nothing early, and 48 mixed frames take 12.7 ms, 13.5 at 40 registers, 13.3 at 32, 12.9 at 64.
@@ -436,9 +425,9 @@ __global__ void WX_RAY_BOUNDS k_persistent(const Job *__restrict__ jobs, uint32_
                     continue;
                 }
             }
-            render_pixel<kModes, true>(J, kBatch == kTableGrid ? tab.g[J.order >> 8] : J.g, t - J.tile_begin + J.tile_off, lane, true);
+            render_pixel<kModes>(J, kBatch == kTableGrid ? tab.g[J.order >> 8] : J.g, t - J.tile_begin + J.tile_off, lane, true);
         } else {
-            render_pixel<kModes, true>(job0, job0.g, t, lane, true);
+            render_pixel<kModes>(job0, job0.g, t, lane, true);
         }
     }
 }
