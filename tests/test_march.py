@@ -117,3 +117,19 @@ def test_large_tile_distances(cuda_ctx, big):
         rg, hg = gpu_render(cuda_ctx, g, st, 96, 96)
         ro, ho = oracle_render(view, st, 96, 96)
         compare(rg, hg, ro, ho, label=f"big {big} mode {mode}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("target", [(1, 1, 1), (-1, 1, 1), (1, -1, 1), (-1, -1, 1), (1, 1, -1), (-1, 1, -1), (1, -1, -1),
+                                    (-1, -1, -1), (0, 1, 0.02), (1, 0, 0.02), (0.02, 0, 1)])
+def test_sign_patterns(cuda_ctx, target):
+    """A loop per sign pattern of the directions, and tiles whose rays differ in it (views along an axis)."""
+    rng = np.random.default_rng(7)
+    topo = wx.Topology.from_voxels(rng.integers(-250, 250, size=(4000, 3)).astype(np.int32))
+    view, g = oracle_view(topo), cuda_ctx.build_grid(topo)
+    for eye, fovy, mode in (((3.0, -5.0, 7.0), 40.0, 3), (tuple(-300.0 * c for c in target), 80.0, 2)):
+        st = wx.state_build(eye=eye, target=tuple(e + 100.0 * c for e, c in zip(eye, target)), aspect=1.5, fovy=fovy,
+                            up=(0.0, 0.3, 1.0), width=120.0, mode=mode)
+        rg, hg = gpu_render(cuda_ctx, g, st, 120, 80)
+        ro, ho = oracle_render(view, st, 120, 80)
+        compare(rg, hg, ro, ho, label=f"{target} mode {mode}")

@@ -47,7 +47,7 @@ __device__ __forceinline__ bool tile_pixel(const Job &J, uint32_t tl, uint32_t l
 
 constexpr int kBase = 1, kGlossy = 2, kSurface = 4, kAllModes = 7;
 
-template <int kModes>
+template <int kModes, bool kOct>
 __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uint32_t tl, uint32_t lane, bool wait_prev,
                                              uint32_t lanes = ~0u) {  // lanes: the warp's lanes that are here
     uint32_t gx, gy;
@@ -74,7 +74,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uin
         if (wx_in_range(pix, (uint64_t)J.width * J.height)) J.rgba[pix] = pack_rgba(c);
         return;
     }
-    const March hit = hdda(G, eye, dir);
+    const March hit = hdda<kOct>(G, eye, dir, kOct ? shared_octant(act, dir) : 8u);
     __syncwarp(act);
     F3 c;
     uint32_t shadow = 0, reserved = 0;
@@ -112,7 +112,8 @@ __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uin
         const uint32_t node = hit.node;
         __syncwarp(act);  // shadow rays of the warp start together
         if (need) {
-            const March sh = hdda(G, src, -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]));
+            const F3 sdir = -f3(s.sun_dir[0], s.sun_dir[1], s.sun_dir[2]);
+            const March sh = hdda<kOct>(G, src, sdir, octant(sdir));
             shadow = 1u | (sh.state << 1) | (sh.i << 8);
             if (sh.state == 0u) cpk = pack_rgba(ambient_colour());  // shadowed is I_a
         }
@@ -139,14 +140,14 @@ __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uin
 // Blocks of at most 256 threads. k_pixel in modes 0-3: 8 resident, 32 registers a thread, all 64
 // warp slots of an SM. Its march waits on dependent loads and leaves a third of its lanes idle, so
 // resident warps pay more than the three reloads an iteration that 32 registers cost: 8 frames of
-// 2000 spheres at 1080p take 3.25 ms at 32 registers, 3.47 at 40 and 3.67 at 47 (2 noise frames at
-// 4K: 2.18, 2.23 and 2.29 ms). The glossy kernel takes 0.38 ms for a 720p frame at 40 and 48
-// registers, 0.39 at 32 and 0.42 at 64; a zero-crossing 1080p frame 0.54 ms at 32, 0.58 at 40 and 0.59
+// 2000 spheres at 1080p take 3.18 ms at 32 registers, 3.3 at 40 and 3.5 at 48 (2 noise frames at
+// 4K: 2.14, 2.15 and 2.19 ms). The glossy kernel takes 0.377 ms for a 720p frame at 48
+// registers, 0.384 at 40, 0.394 at 32 and 0.42 at 64; a zero-crossing 1080p frame 0.54 ms at 32, 0.58 at 40 and 0.59
 // at 48. The persistent kernels keep 48 (5 blocks, 40 warps): their warps live on, so that a finished
 // block frees nothing early, and 48 mixed frames take 12.7 ms, 13.5 at 40 registers, 13.3 at 32, 12.9 at 64.
 // (One warp per tile over the job table instead of the queue: 13.9 ms at 32 registers, 13.5 at 48.)
 #define WX_RAY_BOUNDS __launch_bounds__(256, 5)
-#define WX_PIXEL_BOUNDS __launch_bounds__(256, kModes == kGlossy ? 6 : 8)
+#define WX_PIXEL_BOUNDS __launch_bounds__(256, kModes == kGlossy ? 5 : 8)
 
 // One warp per tile of one frame, tiles in block order (rows in the job's order).
 // Frames on one stream overlap in time: the next k_pixel starts once every block
@@ -167,7 +168,7 @@ __global__ void WX_PIXEL_BOUNDS k_pixel(const __grid_constant__ Job job, uint32_
     asm volatile("griddepcontrol.launch_dependents;");
     const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31u, n = 32u >> split;
     if ((warp >> split) >= ntiles || lane >= n) return;
-    render_pixel<kModes>(job, job.g, warp >> split, (warp & ((1u << split) - 1u)) * n + lane, disjoint == 0u, ~0u >> (32u - n));
+    render_pixel<kModes, kModes == kBase>(job, job.g, warp >> split, (warp & ((1u << split) - 1u)) * n + lane, disjoint == 0u, ~0u >> (32u - n));
 }
 
 // ---------------------------------------------------------------------------
@@ -370,7 +371,7 @@ __global__ void WX_WAVE_BOUNDS k_wave(const __grid_constant__ Job J, uint32_t nt
         if (!__any_sync(~0u, mine)) continue;
         if (mine) {
             const uint32_t *e = slot + k * kWaveWords;
-            const March sh = hdda(J.g, f3(__uint_as_float(e[0]), __uint_as_float(e[1]), __uint_as_float(e[2])), sdir);
+            const March sh = hdda<false>(J.g, f3(__uint_as_float(e[0]), __uint_as_float(e[1]), __uint_as_float(e[2])), sdir);
             wave_shadow_done(J, e, ambient, sh.state, sh.i);
         }
     }
@@ -425,9 +426,9 @@ __global__ void WX_RAY_BOUNDS k_persistent(const Job *__restrict__ jobs, uint32_
                     continue;
                 }
             }
-            render_pixel<kModes>(J, kBatch == kTableGrid ? tab.g[J.order >> 8] : J.g, t - J.tile_begin + J.tile_off, lane, true);
+            render_pixel<kModes, false>(J, kBatch == kTableGrid ? tab.g[J.order >> 8] : J.g, t - J.tile_begin + J.tile_off, lane, true);
         } else {
-            render_pixel<kModes>(job0, job0.g, t, lane, true);
+            render_pixel<kModes, false>(job0, job0.g, t, lane, true);
         }
     }
 }

@@ -414,21 +414,47 @@ __device__ __forceinline__ float rcp_approx(float x) {
 //    exact enough by a factor of 2^9.
 //  * The products and sums of tMax are exact or rounded once, as in ray_step.
 // Bound by instruction issue (81-88% of the slots) at 20 to 29 of 32 lanes, then by the three
-// dependent loads. Against ray_step<false> in the same kernels: about 106 instead of 132 warp
-// instructions an iteration, no root search, and no table load between the lookup and the
-// quotients; 8 frames of 2000 spheres at 1080p 4.64 -> 3.27 ms, 2 noise frames at 4K 2.97 -> 2.20 ms,
-// 48 mixed frames in one batch 18.1 -> 13.0 ms, one 160x120 frame 33 -> 27 us.
-// Tried and slower there: keeping the mask as three bools (3.41 ms for the 8 frames), any form that
-// lets the compiler turn the level blocks into predicated straight-line code (a box test without a
-// branch 3.57 ms, the leaf overflow handled outside the loop 3.77 ms), floor by a second addition
-// instead of FRND (+1%), step01 by compare and select (3.47), a second loop for warps whose
-// directions have one sign pattern (no change).
-__device__ __forceinline__ March hdda(const DevGrid &g, F3 src, F3 dir) {
-    if (ray_needs_careful_step(src, dir) || (g.inside & 2u)) return hdda_general(g, src, dir, 0u, 0u);
-    float px = src.x, py = src.y, pz = src.z;
-    const float ix = __frcp_rn(dir.x), iy = __frcp_rn(dir.y), iz = __frcp_rn(dir.z);
+// dependent loads: about 100 warp instructions an iteration on 2000 spheres and 96 on noise, where
+// ray_step<false> in the same place took 132 and 123, with a root search and a table load between the
+// lookup and the quotients. 8 frames of 2000 spheres at 1080p 4.64 -> 3.18 ms, 2 noise frames at 4K
+// 2.97 -> 2.14 ms, 48 mixed frames in one batch 17.8 -> 12.7 ms.
+// Tried and slower: keeping the mask as three bools or one word (+2%), any form that lets the compiler
+// turn the level blocks into predicated straight-line code (a box test without a branch +9%, the leaf
+// overflow handled outside the loop +15%), floor by a second addition instead of FRND (+1%), size and
+// sign masks for step01 (+5%), two iterations a loop trip (-2% on noise, +4% on the spheres), a dense
+// table of all N3-sized cells around the N4s with a loop of its own inside and outside it (+10%).
+// State of a ray in the loop. t, tx, ty, tz: the last step's mask is tx == t, ty == t, tz == t.
+struct Loop {
+    float px, py, pz;
+    float t, tx, ty, tz;
+    uint32_t lx, ly, lz, scl, i4, i3, i, w;
+};
+
+// One axis of a step: the distance along the ray to the cell's border, idir * (size * step01 - (p - size * f)), with
+// the sign of the direction known (kNeg, kPos) or not. -0 for +0 changes nothing, see ray_step.
+enum Sign { kNeg, kPos, kAny };
+template <Sign kS>
+__device__ __forceinline__ float step01(float d) {
+    return kS == kAny ? __fadd_rn(copysignf(0.5f, d), 0.5f) : 0.0f;  // used where the sign is not known
+}
+template <Sign kS>
+__device__ __forceinline__ float border(float idir, float a, float size, float f, float p) {
+    const float mod = __fmaf_rn(-size, f, p);
+    if (kS == kNeg) return idir * -mod;
+    if (kS == kPos) return idir * (size - mod);
+    return idir * __fmaf_rn(size, a, -mod);
+}
+template <Sign kS>
+__device__ __forceinline__ float nudge(float d) {
+    const float kNudge = 0.5f * 8e-4f;
+    return kS == kNeg ? -kNudge : kS == kPos ? kNudge : copysignf(kNudge, d);
+}
+
+template <Sign kX, Sign kY, Sign kZ>
+__device__ __forceinline__ void march_loop(const DevGrid &g, Loop &s, F3 dir, float ix, float iy, float iz) {
+    float px = s.px, py = s.py, pz = s.pz;
     uint32_t lx = 0, ly = 0, lz = 0, scl = 4096u, i4 = 0, i3 = 0, i = 0, w;
-    float t = 0.0f, tx = 1.0f, ty = 1.0f, tz = 1.0f;  // the last step's mask is tx == t, ty == t, tz == t
+    float t = 0.0f, tx = 1.0f, ty = 1.0f, tz = 1.0f;
     do {
         const float rx = __fadd_rd(px, kFloorMagic), ry = __fadd_rd(py, kFloorMagic), rz = __fadd_rd(pz, kFloorMagic);
         const uint32_t x = __float_as_uint(rx), y = __float_as_uint(ry), z = __float_as_uint(rz);
@@ -459,45 +485,76 @@ __device__ __forceinline__ March hdda(const DevGrid &g, F3 src, F3 dir) {
             if (w == 255u) w = leaf_overflow(g, key);
             scl = 1u;
         }
-        const uint32_t s = w * scl;  // grids with tile distances of 2^24 or more are marched by hdda_general
-        if (s == 0u || min(min(__float_as_int(px), __float_as_int(py)), __float_as_int(pz)) < (int)0x9F800000) break;
-        const float size = __uint2float_rn(s), rc = rcp_approx(size), hf = 0.5f * rc;
-        const float ax = __fadd_rn(copysignf(0.5f, dir.x), 0.5f);
-        const float ay = __fadd_rn(copysignf(0.5f, dir.y), 0.5f);
-        const float az = __fadd_rn(copysignf(0.5f, dir.z), 0.5f);
+        const uint32_t sz = w * scl;  // grids with tile distances of 2^24 or more are marched by hdda_general
+        if (sz == 0u || min(min(__float_as_int(px), __float_as_int(py)), __float_as_int(pz)) < (int)0x9F800000) break;
+        const float size = __uint2float_rn(sz), rc = rcp_approx(size), hf = 0.5f * rc;
+        const float ax = step01<kX>(dir.x), ay = step01<kY>(dir.y), az = step01<kZ>(dir.z);
         const float fx = floorf(__fmaf_rn(rx - kFloorMagic, rc, hf));
         const float fy = floorf(__fmaf_rn(ry - kFloorMagic, rc, hf));
         const float fz = floorf(__fmaf_rn(rz - kFloorMagic, rc, hf));
-        tx = ix * __fmaf_rn(size, ax, -__fmaf_rn(-size, fx, px));
-        ty = iy * __fmaf_rn(size, ay, -__fmaf_rn(-size, fy, py));
-        tz = iz * __fmaf_rn(size, az, -__fmaf_rn(-size, fz, pz));
+        tx = border<kX>(ix, ax, size, fx, px);
+        ty = border<kY>(iy, ay, size, fy, py);
+        tz = border<kZ>(iz, az, size, fz, pz);
         t = fminf(fminf(tx, ty), tz);
         const bool mx = tx == t, my = ty == t, mz = tz == t;
         px = px + t * dir.x;
         py = py + t * dir.y;
         pz = pz + t * dir.z;
-        const float kNudge = 0.5f * 8e-4f;
-        const float nx = copysignf(kNudge, dir.x), ny = copysignf(kNudge, dir.y), nz = copysignf(kNudge, dir.z);
+        const float nx = nudge<kX>(dir.x), ny = nudge<kY>(dir.y), nz = nudge<kZ>(dir.z);
         px = mx ? px + nx : px;
         py = my ? py + ny : py;
         pz = mz ? pz + nz : pz;
     } while (++i < kMaxSteps);
-    const bool mx = tx == t, my = ty == t, mz = tz == t;
+    s = Loop{px, py, pz, t, tx, ty, tz, lx, ly, lz, scl, i4, i3, i, w};
+}
+
+// kOct: a loop for each of the eight sign patterns of a direction, in which step01 and the nudge are constants (8 frames
+// of 2000 spheres 3.25 -> 3.18 ms, 2 noise frames 2.18 -> 2.14 ms; a tile's rays rarely differ). The persistent kernels
+// have rays of several frames on an SM at a time, and nine loops are too much code for them (12.7 -> 13.0 ms); so they
+// are beside the zero-crossing search (0.53 -> 0.57 ms).
+// oct says which direction components are negative (bits x, y, z) for every lane that calls together, or is 8 where they differ.
+template <bool kOct>
+__device__ __forceinline__ March hdda(const DevGrid &g, F3 src, F3 dir, uint32_t oct = 8u) {
+    if (ray_needs_careful_step(src, dir) || (g.inside & 2u)) return hdda_general(g, src, dir, 0u, 0u);
+    Loop s{src.x, src.y, src.z, 0.0f, 1.0f, 1.0f, 1.0f, 0, 0, 0, 4096u, 0, 0, 0, 0};
+    const float ix = __frcp_rn(dir.x), iy = __frcp_rn(dir.y), iz = __frcp_rn(dir.z);
+    if (!kOct) march_loop<kAny, kAny, kAny>(g, s, dir, ix, iy, iz);
+    else switch (oct) {
+        case 0: march_loop<kPos, kPos, kPos>(g, s, dir, ix, iy, iz); break;
+        case 1: march_loop<kNeg, kPos, kPos>(g, s, dir, ix, iy, iz); break;
+        case 2: march_loop<kPos, kNeg, kPos>(g, s, dir, ix, iy, iz); break;
+        case 3: march_loop<kNeg, kNeg, kPos>(g, s, dir, ix, iy, iz); break;
+        case 4: march_loop<kPos, kPos, kNeg>(g, s, dir, ix, iy, iz); break;
+        case 5: march_loop<kNeg, kPos, kNeg>(g, s, dir, ix, iy, iz); break;
+        case 6: march_loop<kPos, kNeg, kNeg>(g, s, dir, ix, iy, iz); break;
+        case 7: march_loop<kNeg, kNeg, kNeg>(g, s, dir, ix, iy, iz); break;
+        default: march_loop<kAny, kAny, kAny>(g, s, dir, ix, iy, iz);
+    }
+    const bool mx = s.tx == s.t, my = s.ty == s.t, mz = s.tz == s.t;
     March m;
     m.mask = (uint32_t)mx | ((uint32_t)my << 1) | ((uint32_t)mz << 2);
-    m.state = i == kMaxSteps ? 2u : w != 0u ? 3u : scl != 4096u ? 0u : 1u;
-    if (m.state == 1u && !(g.inside == 1u && 4096.0f < fmaxf(fmaxf(fabsf(px), fabsf(py)), fabsf(pz)))) m.state = 3u;
-    if (m.state == 3u) return hdda_general(g, f3(px, py, pz), dir, i, m.mask);
-    m.p = f3(px, py, pz);
-    m.i = i;
-    m.np = scl == 1u ? 3u : scl == 8u ? 2u : 0u;
-    m.node = scl == 1u ? i3 >> 9 : scl == 8u ? i4 >> 12 : kNoNode;
-    if (scl == 128u) {  // an N5's slot, or a missing N5
-        m.node = root_find(g, (int)(lx & (kBoxSide - 1u)) - 4096, (int)(ly & (kBoxSide - 1u)) - 4096,
-                           (int)(lz & (kBoxSide - 1u)) - 4096);
+    m.state = s.i == kMaxSteps ? 2u : s.w != 0u ? 3u : s.scl != 4096u ? 0u : 1u;
+    if (m.state == 1u && !(g.inside == 1u && 4096.0f < fmaxf(fmaxf(fabsf(s.px), fabsf(s.py)), fabsf(s.pz)))) m.state = 3u;
+    if (m.state == 3u) return hdda_general(g, f3(s.px, s.py, s.pz), dir, s.i, m.mask);
+    m.p = f3(s.px, s.py, s.pz);
+    m.i = s.i;
+    m.np = s.scl == 1u ? 3u : s.scl == 8u ? 2u : 0u;
+    m.node = s.scl == 1u ? s.i3 >> 9 : s.scl == 8u ? s.i4 >> 12 : kNoNode;
+    if (s.scl == 128u) {  // an N5's slot, or a missing N5
+        m.node = root_find(g, (int)(s.lx & (kBoxSide - 1u)) - 4096, (int)(s.ly & (kBoxSide - 1u)) - 4096,
+                           (int)(s.lz & (kBoxSide - 1u)) - 4096);
         m.np = m.node != kNoNode ? 1u : 0u;
     }
     return m;
+}
+
+__device__ __forceinline__ uint32_t octant(F3 d) {
+    return (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
+}
+// The octant that the directions of the lanes in act share, or 8.
+__device__ __forceinline__ uint32_t shared_octant(uint32_t act, F3 d) {
+    const uint32_t o = octant(d), any = __reduce_or_sync(act, o);
+    return any == __reduce_and_sync(act, o) ? any : 8u;
 }
 
 __device__ __forceinline__ F3 maskf(uint32_t m) {
@@ -529,7 +586,7 @@ __device__ __forceinline__ F3 lit_colour(const DevGrid &g, const wx_state_unifor
     const F3 base = f3(0.4f, 0.2f, 0.2f);
     if (I != 0.0f) {
         const F3 src = h.p - (4e-2f * step) * maskf(h.mask);
-        if (hdda(g, src, -sun).state == 0u) return base + (I * sc) * 0.05f;
+        if (hdda<true>(g, src, -sun, octant(-sun)).state == 0u) return base + (I * sc) * 0.05f;
     }
     return base + I * sc;
 }
@@ -627,7 +684,7 @@ __device__ __forceinline__ F3 glossy_colour(const DevGrid &g, const wx_state_uni
     uint32_t depth = 0;
 #pragma unroll 1
     for (;; depth++) {
-        const March hit = hdda(g, src, dir);
+        const March hit = hdda<false>(g, src, dir);
         if (depth == 0u) first(hit);
         const bool lit = hit.state == 0u;
         act = __ballot_sync(act, lit);
