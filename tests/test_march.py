@@ -93,6 +93,25 @@ def test_rays_at_the_edges_of_the_loop(cuda_ctx, grid, kernel):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("far", [-4198400, -12587008, -4198400 - 2 ** 21, -8392704])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_far_eyes(cuda_ctx, far, axis):
+    """Eyes so far out along one axis that their floor word's high bits are a part of the box's (or all clear),
+    with the other two coordinates in the box: a ray is in the box only if each of its coordinates is."""
+    cube = np.stack(np.mgrid[0:30, 0:30, 0:30], -1).reshape(-1, 3) - 15
+    for extra in ([0, 0, 0], [5000, 10, 20]):
+        topo = wx.Topology.from_voxels(np.concatenate([cube, cube * 9, cube + extra]).astype(np.int32))
+        view, g = oracle_view(topo), cuda_ctx.build_grid(topo)
+        for dist, mode in ((100.0, 3), (700.0, 2)):
+            eye, target = [3.5, 4.5, 5.5], [3.5, 4.5, 5.5]
+            eye[axis], target[axis] = far + 4096 - dist, far + 4096 + 1000.0
+            st = wx.state_build(eye=tuple(eye), target=tuple(target), up=(0.3, 0.5, 0.7), aspect=1.0, fovy=60.0, width=64.0, mode=mode)
+            rg, hg = gpu_render(cuda_ctx, g, st, 64, 64)
+            ro, ho = oracle_render(view, st, 64, 64)
+            compare(rg, hg, ro, ho, label=f"far {far} axis {axis} mode {mode}")
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("big", [2 ** 24 - 1, 2 ** 24, 2 ** 24 + 1, 2 ** 31 - 1])
 def test_large_tile_distances(cuda_ctx, big):
     """Tiles of a hand-made view with distances around the limit of the loop's integer size."""

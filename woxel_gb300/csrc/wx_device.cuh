@@ -464,7 +464,8 @@ __device__ __forceinline__ void march_loop(const DevGrid &g, Loop &s, F3 dir, fl
         if (d >= 128u) {  // get_vdb_leaf_from_nothing / from_node5 (:398-444)
             w = 0u;
             scl = 4096u;
-            if (((x | y | z) ^ kBoxBits) < kBoxSide) {
+            // Each word against the box's bits: the or of x, y and z would also hold them where one of the three does.
+            if (((x ^ kBoxBits) | (y ^ kBoxBits) | (z ^ kBoxBits)) < kBoxSide) {
                 const uint32_t idx = ((x & 0x1F80u) << 5) | ((y >> 1) & 0xFC0u) | ((z >> 7) & 0x3Fu);
                 w = __ldg(g.slot5 - wxk::kTopWords + idx);
                 i4 = w << 12;
