@@ -140,11 +140,11 @@ __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uin
 // Blocks of at most 256 threads. k_pixel in modes 0-3: 8 resident, 32 registers a thread, all 64
 // warp slots of an SM. Its march waits on dependent loads and leaves a third of its lanes idle, so
 // resident warps pay more than the three reloads an iteration that 32 registers cost: 8 frames of
-// 2000 spheres at 1080p take 3.18 ms at 32 registers, 3.3 at 40 and 3.5 at 48 (2 noise frames at
-// 4K: 2.14, 2.15 and 2.19 ms). The glossy kernel takes 0.377 ms for a 720p frame at 48
-// registers, 0.384 at 40, 0.394 at 32 and 0.42 at 64; a zero-crossing 1080p frame 0.54 ms at 32, 0.58 at 40 and 0.59
-// at 48. The persistent kernels keep 48 (5 blocks, 40 warps): their warps live on, so that a finished
-// block frees nothing early, and 48 mixed frames take 12.7 ms, 13.5 at 40 registers, 13.3 at 32, 12.9 at 64.
+// 2000 spheres at 1080p take 3.04 ms at 32 registers, 3.18 at 40 and 3.37 at 48 (2 noise frames at
+// 4K, where nearly all lanes are busy: 2.04, 2.02 and 2.01 ms). The glossy kernel takes 0.368 ms for a 720p
+// frame at 48 registers and at 40, 0.383 at 32 and 0.40 at 64; a zero-crossing 1080p frame 0.525 ms at 32 and
+// 0.55 at 40. The persistent kernels keep 48 (5 blocks, 40 warps): their warps live on, so that a finished
+// block frees nothing early, and 48 mixed frames take 12.48 ms, 12.53 at 40 registers and 12.8 at 32.
 // (One warp per tile over the job table instead of the queue: 13.9 ms at 32 registers, 13.5 at 48.)
 #define WX_RAY_BOUNDS __launch_bounds__(256, 5)
 #define WX_PIXEL_BOUNDS __launch_bounds__(256, kModes == kGlossy ? 5 : 8)

@@ -393,12 +393,50 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return y;
 }
 
+// Two FP32 values in a register pair: one instruction for both (each half rounded as by itself).
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pair(float a, float b) {
+    Pair r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float first(Pair a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return x;
+}
+__device__ __forceinline__ float second(Pair a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return y;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+    Pair r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+    Pair r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair add2(Pair a, Pair b) {
+    Pair r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ Pair add2_ru(Pair a, Pair b) {
+    Pair r;
+    asm("add.rp.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // hdda_ray (raycast.comp.wgsl:84-126) run to completion.
 //
 // The loop below performs the shader's iterations on the rays that need no care
 // (ray_needs_careful_step), with the same results bit for bit; what it does not cover leaves it and
 // is finished by hdda_general from the state reached: a position outside the box [-4096, 4096)^3
-// that does not end the ray, and a coordinate in (-2^-64, 0).
+// that does not end the ray, and a coordinate in (-2^-64, 0) or that became 0 in a step.
 //  * Lookup. Inside the box the N5 slot words of all octants form one dense table (64^3 words before
 //    slot5; 32 fills a missing N5: a tile of 32 * 128 = 4096 voxels, the size an absent N5 has), so a
 //    lookup is at most three loads and needs no root search. scl is the size scale of the level that
@@ -416,13 +454,15 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // Bound by instruction issue (81-88% of the slots) at 20 to 29 of 32 lanes, then by the three
 // dependent loads: about 100 warp instructions an iteration on 2000 spheres and 96 on noise, where
 // ray_step<false> in the same place took 132 and 123, with a root search and a table load between the
-// lookup and the quotients. 8 frames of 2000 spheres at 1080p 4.64 -> 3.18 ms, 2 noise frames at 4K
-// 2.97 -> 2.14 ms, 48 mixed frames in one batch 17.8 -> 12.7 ms.
+// lookup and the quotients. 8 frames of 2000 spheres at 1080p 4.64 -> 3.04 ms, 2 noise frames at 4K
+// 2.97 -> 2.04 ms, 48 mixed frames in one batch 17.8 -> 12.5 ms; of that the pairs gave 3.18 -> 3.04, 2.14 -> 2.04
+// and 12.7 -> 12.5.
 // Tried and slower: keeping the mask as three bools or one word (+2%), any form that lets the compiler
 // turn the level blocks into predicated straight-line code (a box test without a branch +9%, the leaf
 // overflow handled outside the loop +15%), floor by a second addition instead of FRND (+1%), size and
 // sign masks for step01 (+5%), two iterations a loop trip (-2% on noise, +4% on the spheres), a dense
 // table of all N3-sized cells around the N4s with a loop of its own inside and outside it (+10%).
+
 // State of a ray in the loop. t, tx, ty, tz: the last step's mask is tx == t, ty == t, tz == t.
 struct Loop {
     float px, py, pz;
@@ -430,34 +470,36 @@ struct Loop {
     uint32_t lx, ly, lz, scl, i4, i3, i, w;
 };
 
-// One axis of a step: the distance along the ray to the cell's border, idir * (size * step01 - (p - size * f)), with
-// the sign of the direction known (kNeg, kPos) or not. -0 for +0 changes nothing, see ray_step.
-enum Sign { kNeg, kPos, kAny };
-template <Sign kS>
-__device__ __forceinline__ float step01(float d) {
-    return kS == kAny ? __fadd_rn(copysignf(0.5f, d), 0.5f) : 0.0f;  // used where the sign is not known
-}
-template <Sign kS>
-__device__ __forceinline__ float border(float idir, float a, float size, float f, float p) {
-    const float mod = __fmaf_rn(-size, f, p);
-    if (kS == kNeg) return idir * -mod;
-    if (kS == kPos) return idir * (size - mod);
-    return idir * __fmaf_rn(size, a, -mod);
-}
+enum Sign { kNeg, kPos, kAny };  // of a direction component: known, or not
 template <Sign kS>
 __device__ __forceinline__ float nudge(float d) {
     const float kNudge = 0.5f * 8e-4f;
     return kS == kNeg ? -kNudge : kS == kPos ? kNudge : copysignf(kNudge, d);
 }
+template <Sign kS>
+__device__ __forceinline__ float step01(float d) {
+    return kS == kNeg ? 0.0f : kS == kPos ? 1.0f : __fadd_rn(copysignf(0.5f, d), 0.5f);
+}
 
+// The loop on q = -p, x and y in pairs. Negated, each term of a step is one operation: rounding -p - kFloorMagic up gives
+// minus the rounded-down sum (the same bits but for the sign), size * f + q is -(p - size * f), and size * step01 added to
+// that is the distance to the border. Rounding to nearest is symmetric, so all values are those of the shader's order. The
+// sign of a zero may differ: no step depends on it, a q of +0 leaves the loop with the small ones, and 0 - q makes it +0
+// again (p is never -0 on these rays). The products of q's step are scalar: with a paired product ptxas 13.0 contracts it
+// and the sum into one fma, whatever their rounding modifiers say (positions off by an ulp).
 template <Sign kX, Sign kY, Sign kZ>
 __device__ __forceinline__ void march_loop(const DevGrid &g, Loop &s, F3 dir, float ix, float iy, float iz) {
-    float px = s.px, py = s.py, pz = s.pz;
+    Pair q = pair(-s.px, -s.py);
+    float qz = -s.pz;
+    const Pair nd = pair(-dir.x, -dir.y), id = pair(ix, iy);
     uint32_t lx = 0, ly = 0, lz = 0, scl = 4096u, i4 = 0, i3 = 0, i = 0, w;
-    float t = 0.0f, tx = 1.0f, ty = 1.0f, tz = 1.0f;
+    float t = 0.0f, tz = 1.0f;
+    Pair txy = pair(1.0f, 1.0f);
+    constexpr uint32_t kNegBox = 0x80000000u | kBoxBits;
     do {
-        const float rx = __fadd_rd(px, kFloorMagic), ry = __fadd_rd(py, kFloorMagic), rz = __fadd_rd(pz, kFloorMagic);
-        const uint32_t x = __float_as_uint(rx), y = __float_as_uint(ry), z = __float_as_uint(rz);
+        const Pair r = add2_ru(q, pair(-kFloorMagic, -kFloorMagic));
+        const float rz = __fadd_ru(qz, -kFloorMagic);
+        const uint32_t x = __float_as_uint(first(r)), y = __float_as_uint(second(r)), z = __float_as_uint(rz);
         const uint32_t d = (x ^ lx) | (y ^ ly) | (z ^ lz) | scl;
         lx = x; ly = y; lz = z;
         w = kChild;
@@ -465,7 +507,7 @@ __device__ __forceinline__ void march_loop(const DevGrid &g, Loop &s, F3 dir, fl
             w = 0u;
             scl = 4096u;
             // Each word against the box's bits: the or of x, y and z would also hold them where one of the three does.
-            if (((x ^ kBoxBits) | (y ^ kBoxBits) | (z ^ kBoxBits)) < kBoxSide) {
+            if (((x ^ kNegBox) | (y ^ kNegBox) | (z ^ kNegBox)) < kBoxSide) {
                 const uint32_t idx = ((x & 0x1F80u) << 5) | ((y >> 1) & 0xFC0u) | ((z >> 7) & 0x3Fu);
                 w = __ldg(g.slot5 - wxk::kTopWords + idx);
                 i4 = w << 12;
@@ -487,32 +529,39 @@ __device__ __forceinline__ void march_loop(const DevGrid &g, Loop &s, F3 dir, fl
             scl = 1u;
         }
         const uint32_t sz = w * scl;  // grids with tile distances of 2^24 or more are marched by hdda_general
-        if (sz == 0u || min(min(__float_as_int(px), __float_as_int(py)), __float_as_int(pz)) < (int)0x9F800000) break;
-        const float size = __uint2float_rn(sz), rc = rcp_approx(size), hf = 0.5f * rc;
-        const float ax = step01<kX>(dir.x), ay = step01<kY>(dir.y), az = step01<kZ>(dir.z);
-        const float fx = floorf(__fmaf_rn(rx - kFloorMagic, rc, hf));
-        const float fy = floorf(__fmaf_rn(ry - kFloorMagic, rc, hf));
-        const float fz = floorf(__fmaf_rn(rz - kFloorMagic, rc, hf));
-        tx = border<kX>(ix, ax, size, fx, px);
-        ty = border<kY>(iy, ay, size, fy, py);
-        tz = border<kZ>(iz, az, size, fz, pz);
+        if (sz == 0u || min(min(__float_as_uint(first(q)), __float_as_uint(second(q))), __float_as_uint(qz)) < 0x1F800000u) break;
+        const float size = __uint2float_rn(sz), nrc = -rcp_approx(size);
+        const Pair size2 = pair(size, size), rc2 = pair(nrc, nrc), hf = mul2(rc2, pair(-0.5f, -0.5f));
+        const Pair v = fma2(add2(r, pair(kFloorMagic, kFloorMagic)), rc2, hf);
+        const float vz = __fmaf_rn(rz + kFloorMagic, nrc, first(hf));
+        const Pair f = pair(floorf(first(v)), floorf(second(v)));
+        Pair m = fma2(size2, f, q);
+        float mz = __fmaf_rn(size, floorf(vz), qz);
+        if (kX == kPos && kY == kPos) m = add2(size2, m);
+        else if (!(kX == kNeg && kY == kNeg)) m = fma2(size2, pair(step01<kX>(dir.x), step01<kY>(dir.y)), m);
+        if (kZ == kPos) mz = size + mz;
+        else if (kZ == kAny) mz = __fmaf_rn(size, step01<kZ>(dir.z), mz);
+        txy = mul2(id, m);
+        tz = iz * mz;
+        const float tx = first(txy), ty = second(txy);
         t = fminf(fminf(tx, ty), tz);
-        const bool mx = tx == t, my = ty == t, mz = tz == t;
-        px = px + t * dir.x;
-        py = py + t * dir.y;
-        pz = pz + t * dir.z;
+        const bool bx = tx == t, by = ty == t, bz = tz == t;
+        q = add2(q, pair(__fmul_rn(t, first(nd)), __fmul_rn(t, second(nd))));
+        qz = qz + t * -dir.z;
         const float nx = nudge<kX>(dir.x), ny = nudge<kY>(dir.y), nz = nudge<kZ>(dir.z);
-        px = mx ? px + nx : px;
-        py = my ? py + ny : py;
-        pz = mz ? pz + nz : pz;
+        float qx = first(q), qy = second(q);
+        qx = bx ? qx - nx : qx;
+        qy = by ? qy - ny : qy;
+        qz = bz ? qz - nz : qz;
+        q = pair(qx, qy);
     } while (++i < kMaxSteps);
-    s = Loop{px, py, pz, t, tx, ty, tz, lx, ly, lz, scl, i4, i3, i, w};
+    s = Loop{0.0f - first(q), 0.0f - second(q), 0.0f - qz, t, first(txy), second(txy), tz, lx, ly, lz, scl, i4, i3, i, w};
 }
 
 // kOct: a loop for each of the eight sign patterns of a direction, in which step01 and the nudge are constants (8 frames
-// of 2000 spheres 3.25 -> 3.18 ms, 2 noise frames 2.18 -> 2.14 ms; a tile's rays rarely differ). The persistent kernels
-// have rays of several frames on an SM at a time, and nine loops are too much code for them (12.7 -> 13.0 ms); so they
-// are beside the zero-crossing search (0.53 -> 0.57 ms).
+// of 2000 spheres 3.11 -> 3.04 ms, 2 noise frames 2.09 -> 2.04 ms; a tile's rays rarely differ). The persistent kernels
+// have rays of several frames on an SM at a time, and nine loops are too much code for them (12.5 -> 12.9 ms); so they
+// are beside the zero-crossing search (0.525 -> 0.56 ms).
 // oct says which direction components are negative (bits x, y, z) for every lane that calls together, or is 8 where they differ.
 template <bool kOct>
 __device__ __forceinline__ March hdda(const DevGrid &g, F3 src, F3 dir, uint32_t oct = 8u) {
