@@ -485,8 +485,11 @@ __device__ __forceinline__ float step01(float d) {
 // minus the rounded-down sum (the same bits but for the sign), size * f + q is -(p - size * f), and size * step01 added to
 // that is the distance to the border. Rounding to nearest is symmetric, so all values are those of the shader's order. The
 // sign of a zero may differ: no step depends on it, a q of +0 leaves the loop with the small ones, and 0 - q makes it +0
-// again (p is never -0 on these rays). The products of q's step are scalar: with a paired product ptxas 13.0 contracts it
-// and the sum into one fma, whatever their rounding modifiers say (positions off by an ulp).
+// again (p is never -0 on these rays). A source coordinate of 0 is -0 here and must not become +0 in the first step, or an
+// eye on an axis plane would have its rays marched by hdda_general (a 640x480 frame of one sphere from there 50 -> 71 us):
+// with the distance t to its border +0 and not -0, it stays -0 where the direction is positive, and is nudged elsewhere.
+// The products of q's step are scalar: with a paired product ptxas 13.0 contracts it and the sum into one fma, whatever
+// their rounding modifiers say (positions off by an ulp).
 template <Sign kX, Sign kY, Sign kZ>
 __device__ __forceinline__ void march_loop(const DevGrid &g, Loop &s, F3 dir, float ix, float iy, float iz) {
     Pair q = pair(-s.px, -s.py);
@@ -541,8 +544,8 @@ __device__ __forceinline__ void march_loop(const DevGrid &g, Loop &s, F3 dir, fl
         else if (!(kX == kNeg && kY == kNeg)) m = fma2(size2, pair(step01<kX>(dir.x), step01<kY>(dir.y)), m);
         if (kZ == kPos) mz = size + mz;
         else if (kZ == kAny) mz = __fmaf_rn(size, step01<kZ>(dir.z), mz);
-        txy = mul2(id, m);
-        tz = iz * mz;
+        txy = fma2(id, m, pair(0.0f, 0.0f));  // + 0: a distance of 0 is +0, see above
+        tz = __fmaf_rn(iz, mz, 0.0f);
         const float tx = first(txy), ty = second(txy);
         t = fminf(fminf(tx, ty), tz);
         const bool bx = tx == t, by = ty == t, bz = tz == t;
