@@ -165,8 +165,8 @@ int wx_grid_build(wx_ctx *ctx, wx_topology *topo, wx_grid **out);
  * vdb345.rs:290-670): the same device pools word for word. Needs N5 origins
  * that are multiples of 4096 (else WX_ERR_UNSUPPORTED). Temporary device
  * memory: about 840 bytes per leaf, 23 KB per N4 and 185 KB per N5.
- * The distances are computed in steps, with a barrier of all CTAs between two
- * steps; a CTA waiting there polls at most the context's SDF wait limit
+ * The distances are computed in steps, with a barrier between two steps for the
+ * CTAs that have started; a CTA waiting there polls at most the context's SDF wait limit
  * (wx_ctx_set_sdf_wait_limit) times, then sets an error flag on which every
  * CTA returns: the call then returns WX_ERR_TIMEOUT, builds no grid and leaves
  * the context usable. */

@@ -52,7 +52,7 @@ struct wx_ctx {
     size_t jobs_cap = 0;
     wxk::Job *jobs_host = nullptr;      // pinned staging for that table
     cudaEvent_t jobs_done = nullptr;    // last one-shot batch's table copy
-    uint32_t sdf_spins = wxk::kSdfSpinLimit;  // bound of the GPU SDF sweeps' dependency waits
+    uint32_t sdf_spins = wxk::kSdfSpinLimit;  // bound of the waits in the GPU SDF's step control
     uint32_t *take_counter() {
         uint32_t *c = counters + next_counter;
         next_counter = (next_counter + 1) % kCounterSlots;
@@ -733,7 +733,7 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
             first[l] = carve(nodes[l] * 4);
             cidx[l] = carve(words[l] * 64 * 4);
         }
-        const size_t at_root = carve(root.size() * 16), at_ctl = carve(64);
+        const size_t at_root = carve(root.size() * 16), at_ctl = carve(sizeof(wxk::SdfCtl));
         WX_CUDA(ctx, wx::dev_alloc(&tmp.p, need));
         char *const base = static_cast<char *>(tmp.p);
         auto u64 = [&](size_t at) { return reinterpret_cast<uint64_t *>(base + at); };
@@ -755,9 +755,8 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
         for (auto &u : ups)
             if (u.bytes) WX_CUDA(ctx, cudaMemcpy(base + u.at, u.src, u.bytes, cudaMemcpyHostToDevice));
         const cudaStream_t st = nullptr;
-        uint32_t *const ctl = u32(at_ctl);
-        auto *const left = reinterpret_cast<unsigned long long *>(base + at_ctl + 32);
-        WX_CUDA(ctx, cudaMemsetAsync(ctl, 0, 64, st));
+        auto *const ctl = reinterpret_cast<wxk::SdfCtl *>(base + at_ctl);
+        WX_CUDA(ctx, cudaMemsetAsync(ctl, 0, sizeof *ctl, st));
         WX_CUDA(ctx, wxk::sdf_child_table(u64(z[0]), u32(pre[0]), u32(first[0]), n5, 15, u32(cidx[0]), st));
         WX_CUDA(ctx, wxk::sdf_child_table(u64(z[1]), u32(pre[1]), u32(first[1]), n4, 12, u32(cidx[1]), st));
         WX_CUDA(ctx, wxk::sdf_child_origins(u32(cidx[0]), i4(org[0]), n5, 5, 7, i4(org[1]), st));
@@ -773,25 +772,21 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
                 // The missing neighbour's ones, in z and the W sets.
                 WX_CUDA(ctx, cudaMemset2DAsync(base + z[l] + real, set, 0xFF, set - real, wxk::kSdfWindow + 1, st));
             }
-            WX_CUDA(ctx, wxk::sdf_count_clear(u64(z[l]), words[l], left + l, st));
+            WX_CUDA(ctx, wxk::sdf_count_clear(u64(z[l]), words[l], &ctl->left[l], st));
             work.lv[l] = wxk::SdfLevel{u64(z[l]), (uint32_t)(set / 8), l < 2 ? u64(val[l]) : nullptr, u32(nb[l]), u32(act[l]),
                                        l < 2 ? slots[l] : nullptr, (uint32_t)nodes[l]};
         }
-        WX_CUDA(ctx, cudaMemcpyAsync(left + 3, left + 2, 8, cudaMemcpyDeviceToDevice, st));
+        WX_CUDA(ctx, cudaMemcpyAsync(&ctl->inactive, &ctl->left[2], 8, cudaMemcpyDeviceToDevice, st));
         work.leaf = const_cast<uint8_t *>(gr->g.leaf);
         work.ctl = ctl;
-        work.left = left;
         // Distances below 255 first; the leaf cells then left are the overflow entries.
-        struct {
-            uint32_t ctl[8];
-            unsigned long long left[4];  // [3] the inactive leaf cells, as counted at the start
-        } h;
+        wxk::SdfCtl h;
         WX_CUDA(ctx, wxk::sdf_levels(work, 1, wxk::kSdfWindow, ctx->num_sms, ctx->sdf_spins, st));
         WX_CUDA(ctx, wxk::sdf_expand(work, u32(cidx[0]), u32(cidx[1]), st));
         WX_CUDA(ctx, wxk::sdf_levels(work, wxk::kSdfWindow + 1, 254, ctx->num_sms, ctx->sdf_spins, st));
         WX_CUDA(ctx, wxk::build_top_table(gr->g, st));
         WX_CUDA(ctx, cudaMemcpy(&h, ctl, sizeof h, cudaMemcpyDeviceToHost));
-        if (!h.ctl[2] && (h.left[0] | h.left[1] | h.left[2])) {
+        if (!h.error && (h.left[0] | h.left[1] | h.left[2])) {
             const uint64_t n_ovf = h.left[2];
             if (n_ovf && (rc = alloc_overflow(ctx, gr, n_ovf)) != WX_OK) return rc;
             work.ovf = gr->ovf;
@@ -799,11 +794,11 @@ int wx_grid_build_gpu(wx_ctx *ctx, const wx_topology *t, wx_grid **out) {
             WX_CUDA(ctx, wxk::sdf_levels(work, 255, wxk::kSdfMaxLevel, ctx->num_sms, ctx->sdf_spins, st));
             WX_CUDA(ctx, wxk::build_top_table(gr->g, st));
             WX_CUDA(ctx, cudaMemcpy(&h, ctl, sizeof h, cudaMemcpyDeviceToHost));
-            if (n_ovf && !h.ctl[2] && (rc = sort_overflow(ctx, gr)) != WX_OK) return rc;
+            if (n_ovf && !h.error && (rc = sort_overflow(ctx, gr)) != WX_OK) return rc;
         }
-        if (h.ctl[2]) return fail(ctx, WX_ERR_TIMEOUT, "wx_grid_build_gpu: the distance steps' barrier wait hit its bound");
+        if (h.error) return fail(ctx, WX_ERR_TIMEOUT, "wx_grid_build_gpu: the distance steps' barrier wait hit its bound");
         if (h.left[0] | h.left[1] | h.left[2]) return fail(ctx, WX_ERR_UNSUPPORTED, "wx_grid_build_gpu: distances above 4095");
-        gr->info.active_voxels = n3 * kN3Slots - h.left[3];
+        gr->info.active_voxels = n3 * kN3Slots - h.inactive;
         guard.g = nullptr;
         *out = gr;
         return WX_OK;

@@ -27,7 +27,7 @@
 // same time, on bit masks, 64 cells an instruction.
 //
 // k_sdf_levels advances all nodes of all three levels by one k between two
-// barriers of a cooperative grid. The first kSdfWindow steps, in which all but a
+// barriers of its running CTAs (sdf_steps.h). The first kSdfWindow steps, in which all but a
 // few cells of a level set get their distance, advance every node, keep their W
 // masks, and store nothing else: k_expand_* then turns the masks into pool words,
 // each written once. Later steps alternate between two masks, advance a node only
@@ -46,6 +46,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 
 #include "wx_kernels.h"
@@ -309,7 +310,7 @@ __device__ __forceinline__ uint32_t leaf_step(const SdfWork &S, uint32_t k, uint
         atomicOr(out + y, ((((t & kLow7) + kLow7) | t) >> 7 & kOnes) * byte);
         if (k >= 255u)
             for (uint32_t m = (uint32_t)row; m; m &= m - 1u) {
-                const uint32_t p = atomicAdd(S.ctl + 3, 1u);
+                const uint32_t p = atomicAdd(&S.ctl->n_ovf, 1u);
                 if (p < S.ovf_cap) S.ovf[p] = make_uint2(i * 64u + y * 8u + (uint32_t)__ffs(m) - 1u, k);
             }
     }
@@ -352,11 +353,20 @@ __device__ __forceinline__ uint32_t node_step(const SdfWork &S, uint32_t k, uint
     return __popcll(add);
 }
 
-// Steps k0 to k1, or fewer when every cell has its distance. ctl: [0] arrivals at the barrier, [1] its release
-// (8k + a bit for each of N5, N4, leaves that is done), [2] error flag, [3] overflow entries, [4..6] last step of
-// N5, N4, leaves; left: cells of N5, N4 and
-// leaves without a distance. A level takes no part once none is left in it. A cooperative launch: the CTAs wait for
-// one another.
+// The step control's memory operations (sdf_steps.h).
+struct StepsMem {
+    template <class T>
+    __device__ __forceinline__ T add(T *p, T v) const { return atomicAdd(p, v); }
+    __device__ __forceinline__ uint32_t load(const uint32_t *p) const { return ld_relaxed(p); }
+    __device__ __forceinline__ unsigned long long load(unsigned long long *p) const { return atomicAdd(p, 0ull); }
+    __device__ __forceinline__ void store(uint32_t *p, uint32_t v) const { atomicExch(p, v); }
+    __device__ __forceinline__ void fence() const { __threadfence(); }
+    // Polls are relaxed: an acquire would empty the SM's L1 under the CTAs still at work (the fence after them acquires).
+    __device__ __forceinline__ void pause() const { __nanosleep(256); }
+};
+
+// Steps k0 to k1, or fewer when every cell has its distance. A level takes no part once none is left in it. The CTAs
+// that run share each step among them (sdf_steps.h).
 constexpr uint32_t kLeafChunk = 8;  // groups of three leaves a warp takes at a time, looked over with one load
 // Bound by the latency of its gathers. 2000-sphere grid, 14 steps: 0.76 ms with the two k_expand_* another 0.14 ms; as
 // one kernel that stored every distance by an atomic and marked the neighbours of every change from the first step on,
@@ -364,15 +374,15 @@ constexpr uint32_t kLeafChunk = 8;  // groups of three leaves a warp takes at a 
 // the whole build; 2.04 at 4 CTAs (64 registers), 2.14 at 5, 2.47 at 8 (spills).
 __global__ void __launch_bounds__(256, 6) k_sdf_levels(const __grid_constant__ SdfWork S, uint32_t k0, uint32_t k1,
                                                     uint32_t spin_limit) {
-    __shared__ uint32_t s_new[3], s_done;
-    const uint32_t lane = threadIdx.x & 31u, warp = blockIdx.x * 8u + (threadIdx.x >> 5), warps = gridDim.x * 8u;
+    __shared__ uint32_t s_new[3], s_word, s_ticket;
+    const uint32_t lane = threadIdx.x & 31u;
     const uint32_t n5 = S.lv[0].n * (Geo<5>::kNode / 32), n4 = S.lv[1].n * (Geo<4>::kNode / 32), n3 = S.lv[2].n;
-    if (threadIdx.x == 0u)
-        s_done = S.ctl[2] ? 7u : (S.left[0] == 0ull ? 1u : 0u) | (S.left[1] == 0ull ? 2u : 0u) | (S.left[2] == 0ull ? 4u : 0u);
+    if (threadIdx.x == 0u) s_word = wxk::steps_enter(StepsMem{}, S.ctl, gridDim.x, k0, k1, spin_limit, &s_ticket);
     __syncthreads();
-    for (uint32_t k = k0; k <= k1; k++) {
-        const uint32_t done = s_done;
-        if (done == 7u) return;
+    for (;;) {
+        const uint32_t word = s_word, done = wxk::steps_done(word), k = wxk::steps_k(word) + 1u;
+        if (done == wxk::kStepsAllDone || k > k1) return;
+        const uint32_t warp = s_ticket * 8u + (threadIdx.x >> 5), warps = wxk::steps_ctas(word) * 8u;
         if (threadIdx.x < 3u) s_new[threadIdx.x] = 0;
         __syncthreads();
         uint32_t got[3] = {0, 0, 0};
@@ -395,32 +405,8 @@ __global__ void __launch_bounds__(256, 6) k_sdf_levels(const __grid_constant__ S
         __syncthreads();
         if (threadIdx.x == 0u) {
             for (int l = 0; l < 3; l++)
-                if (s_new[l]) atomicAdd(S.left + l, 0ull - s_new[l]);
-            __threadfence();
-            uint32_t v;
-            if (atomicAdd(S.ctl, 1u) == gridDim.x * (k - k0 + 1u) - 1u) {
-                __threadfence();
-                v = 8u * k;
-                for (uint32_t l = 0; l < 3u; l++) {
-                    v |= atomicAdd(S.left + l, 0ull) == 0ull ? 1u << l : 0u;
-                    if (!((done >> l) & 1u)) S.ctl[4u + l] = k;
-                }
-                atomicExch(S.ctl + 1, v);
-            } else {
-                for (uint32_t polls = 1;; polls++) {
-                    // Relaxed: an acquire would empty the SM's L1 under the CTAs still at work (the fence below acquires).
-                    v = ld_relaxed(S.ctl + 1);
-                    if (v >= 8u * k) break;
-                    if (polls >= spin_limit || ld_relaxed(S.ctl + 2) != 0u) {  // every CTA then returns
-                        atomicExch(S.ctl + 2, 1u);
-                        v = 7u;
-                        break;
-                    }
-                    __nanosleep(256);
-                }
-            }
-            s_done = v & 7u;
-            __threadfence();
+                if (s_new[l]) atomicAdd(&S.ctl->left[l], 0ull - s_new[l]);
+            s_word = wxk::steps_next(StepsMem{}, S.ctl, s_ticket, word, k1, spin_limit);
         }
         __syncthreads();
     }
@@ -436,7 +422,7 @@ __global__ void __launch_bounds__(256) k_expand_leaves(const __grid_constant__ S
     const SdfLevel &V = S.lv[2];
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;
     if (i >= V.n * 8u) return;
-    const uint32_t last = min(S.ctl[6], wxk::kSdfWindow);
+    const uint32_t last = min(S.ctl->last[2], wxk::kSdfWindow);
     uint64_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, w = 0;
     for (uint32_t k = 0; k <= last; k++) {
         w = V.sets[k * V.stride + i];
@@ -470,7 +456,7 @@ __global__ void __launch_bounds__(256) k_expand_nodes(const __grid_constant__ Sd
                                                       const uint4 *__restrict__ cidx) {
     const SdfLevel &V = S.lv[level];
     const uint64_t i = (uint64_t)blockIdx.x * 256u + threadIdx.x;  // grid: exactly a quarter of the level's slots
-    const uint32_t word = (uint32_t)(i >> 4), bit = (uint32_t)(i & 15u) * 4u, last = min(S.ctl[4 + level], wxk::kSdfWindow);
+    const uint32_t word = (uint32_t)(i >> 4), bit = (uint32_t)(i & 15u) * 4u, last = min(S.ctl->last[level], wxk::kSdfWindow);
     const uint32_t kid = (uint32_t)(V.sets[word] >> bit) & 15u, val = (uint32_t)(V.val[word] >> bit) & 15u;
     uint32_t in = kid, d = 0;  // a byte a slot
     auto bytes = [](uint32_t nibble) { return (nibble * 0x00204081u) & 0x01010101u; };
@@ -537,15 +523,15 @@ cudaError_t sdf_neighbours(int level, const int4 *org, uint32_t nc, const SdfTre
 }
 
 cudaError_t sdf_levels(const SdfWork &w, uint32_t k0, uint32_t k1, int num_sms, uint32_t spin_limit, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(w.ctl, 0, 2 * sizeof(uint32_t), st);
+    static_assert(kSdfMaxLevel < 4096u && offsetof(SdfCtl, error) == 16, "steps_word; the part cleared here");
+    cudaError_t e = cudaMemsetAsync(w.ctl, 0, offsetof(SdfCtl, error), st);
     if (e != cudaSuccess) return e;
     const uint64_t tasks = (uint64_t)w.lv[0].n * (Geo<5>::kNode / 32) + (uint64_t)w.lv[1].n * (Geo<4>::kNode / 32) +
                            (w.lv[2].n + 3u * kLeafChunk - 1u) / (3u * kLeafChunk);
-    const uint64_t blocks = std::min<uint64_t>((uint64_t)resident_blocks(k_sdf_levels, 256, 0) * num_sms, (tasks + 7) / 8);
-    SdfWork work = w;
-    void *args[] = {&work, &k0, &k1, &spin_limit};
-    return cudaLaunchCooperativeKernel((const void *)k_sdf_levels, dim3((unsigned)std::max<uint64_t>(blocks, 1)), dim3(256),
-                                       args, 0, st);
+    // As many CTAs as fit the chip; fewer may run (sdf_steps.h).
+    const uint64_t blocks = std::min({(uint64_t)resident_blocks(k_sdf_levels, 256, 0) * num_sms, (tasks + 7) / 8, (uint64_t)kStepsMaxCtas});
+    k_sdf_levels<<<(unsigned)std::max<uint64_t>(blocks, 1), 256, 0, st>>>(w, k0, k1, spin_limit);
+    return cudaGetLastError();
 }
 
 cudaError_t sdf_expand(const SdfWork &w, const uint32_t *cidx5, const uint32_t *cidx4, cudaStream_t st) {

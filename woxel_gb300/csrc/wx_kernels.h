@@ -5,6 +5,7 @@
 
 #include <cstdint>
 
+#include "sdf_steps.h"
 #include "woxel_gb300.h"
 
 namespace wxk {
@@ -88,7 +89,7 @@ bool grid_device_view(const wx_grid *grid, DevGrid *out, int *device);
 // Device index and SM count of a context (defined in api.cpp).
 void ctx_device_info(const wx_ctx *ctx, int *device, int *num_sms);
 
-// GPU SDF build (sdf.cu). The tree structure the sweeps look neighbours up in:
+// GPU SDF build (sdf.cu). The tree structure that neighbours are looked up in:
 // the root block of the grid layout (header, origins, root-key table) and the
 // child-index tables (slot -> child DFS index or 0xFFFFFFFF).
 struct SdfTree {
@@ -125,10 +126,9 @@ struct SdfWork {
     uint8_t *leaf;           // leaf bytes
     uint2 *ovf;              // (cell, distance) of distances >= 255
     uint32_t ovf_cap;
-    uint32_t *ctl;           // 7 words: barrier arrivals and release, error flag, overflow entries, last steps
-    unsigned long long *left;  // cells of N5, N4 and leaves without a distance
+    SdfCtl *ctl;
 };
-// Steps k0..k1 (fewer when *left reaches 0). ctl[2] is set when a wait hit its bound.
+// Steps k0..k1 (fewer when no cell is left). ctl->error is set when a wait hit its bound.
 // spin_limit: polls (256 ns apart) a CTA makes at the barrier between two steps before it sets
 // the error flag and every CTA returns.
 constexpr uint32_t kSdfSpinLimit = 1u << 23;  // about 2 s
