@@ -177,14 +177,16 @@ void *pinned_device_alias(void *p) {
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
-// A device allocation freed on scope exit (temporaries of wx_grid_build_gpu).
+// A device allocation freed on scope exit (temporaries of wx_grid_build_gpu and wx_grid_upload).
 struct DevBuf {
     void *p = nullptr;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    ~DevBuf() {
+    ~DevBuf() { release(); }
+    void release() {
         if (p) cudaFree(p);
+        p = nullptr;
     }
     template <class T>
     T *as() const {
@@ -852,42 +854,40 @@ int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *v, wx_grid **out) {
             const int32_t *o = v->origins + i * v->origin_stride;
             o5[i] = make_int4(o[0], o[1], o[2], 0);
         }
-        // The masks and, slab by slab, the atlases are copied to the device and packed there (pack.cu). A slab is a
-        // layer of d * d nodes (D texel layers, contiguous); the buffer holds as many as fit 256 MB, at least one.
+        // Piece by piece, an atlas and its nodes' masks are copied to the device and packed there (pack.cu). A piece is whole
+        // layers of d * d nodes, or block rows (d nodes) of one layer: as many as fit the buffer, 256 MB where the
+        // device has that beside the grid, less where it has not, down to one block row.
+        const uint32_t *const kids[3] = {v->kids5, v->kids4, nullptr}, *const vals[3] = {v->vals5, v->vals4, v->vals3};
         struct Atlas {
-            int level;
-            uint64_t n, layers, per_buffer;
-            uint32_t d;
-            size_t layer_bytes;
-        } atlas[3] = {{5, n5, 0, 0, d5, 0}, {4, n4, 0, 0, d4, 0}, {3, n3, 0, 0, d3, 0}};
-        size_t slab = 0;
+            uint64_t n, rows;
+            uint32_t d, log2, words;          // mask words of a node
+            size_t texel_row, slice, row;     // bytes: texels of a block row; one texel layer; a block row with its masks
+        } atlas[3] = {{n5, 0, d5, 5, 1024, 0, 0, 0}, {n4, 0, d4, 4, 128, 0, 0, 0}, {n3, 0, d3, 3, 16, 0, 0, 0}};
+        constexpr size_t kFixed = 1024;  // counters and alignment
+        size_t least = kFixed, most = kFixed;
         for (int l = 0; l < 3; l++) {
             Atlas &a = atlas[l];
             if (!a.n) continue;
-            const uint64_t per = (uint64_t)a.d * a.d;
-            a.layers = (a.n + per - 1) / per;
-            a.layer_bytes = ((size_t)v->dims[l][0] * v->dims[l][1] << a.level) * 4;
-            a.per_buffer = std::min<uint64_t>(a.layers, std::max<uint64_t>(1, ((size_t)256 << 20) / a.layer_bytes));
-            slab = std::max(slab, (size_t)a.per_buffer * a.layer_bytes);
-        }
-        const size_t words[5] = {n5 * 1024, n5 * 1024, n4 * 128, n4 * 128, n3 * 16};
-        const uint32_t *const src[5] = {v->kids5, v->vals5, v->kids4, v->vals4, v->vals3};
-        size_t at[5], need = 256;  // 256 bytes of counters
-        for (int i = 0; i < 5; i++) {
-            at[i] = need;
-            need += (words[i] * 4 + 255) & ~(size_t)255;
-        }
-        DevBuf tmp;
-        WX_CUDA(ctx, wx::dev_alloc(&tmp.p, need + slab));
-        char *const base = static_cast<char *>(tmp.p);
-        const uint32_t *mask[5];
-        for (int i = 0; i < 5; i++) {
-            mask[i] = reinterpret_cast<const uint32_t *>(base + at[i]);
-            if (words[i]) WX_CUDA(ctx, cudaMemcpy(base + at[i], src[i], words[i] * 4, cudaMemcpyHostToDevice));
+            a.rows = (a.n + a.d - 1) / a.d;
+            a.texel_row = (size_t)v->dims[l][0] << (2 * a.log2 + 2);
+            a.slice = (size_t)v->dims[l][0] * v->dims[l][1] * 4;
+            a.row = a.texel_row + std::min<uint64_t>(a.n, a.d) * a.words * (kids[l] ? 8 : 4);
+            least = std::max(least, kFixed + a.row);
+            most = std::max(most, kFixed + a.row * (a.rows < a.d ? a.rows : (a.rows + a.d - 1) / a.d * a.d));
         }
         wx_grid *gr = nullptr;
-        if ((rc = alloc_grid(ctx, o5, n5, n4, n3, 0, &gr)) != WX_OK) return rc;
+        DevBuf tmp;
+        size_t bytes = std::max(least, std::min(most, (size_t)256 << 20));
+        for (;; bytes = std::max(least, bytes / 2)) {
+            const cudaError_t e = wx::dev_alloc(&tmp.p, bytes);
+            rc = e == cudaSuccess ? alloc_grid(ctx, o5, n5, n4, n3, 0, &gr) : cuda_fail(ctx, e, "cudaMalloc(upload buffer)");
+            if (rc == WX_OK) break;
+            tmp.release();
+            if (rc != WX_ERR_OOM || bytes == least) return rc;
+            cudaGetLastError();
+        }
         GridGuard guard{gr};
+        char *const base = static_cast<char *>(tmp.p);
         const cudaStream_t st = nullptr;
         struct Counts {
             unsigned long long n_ovf, clear;
@@ -896,25 +896,53 @@ int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *v, wx_grid **out) {
         WX_CUDA(ctx, cudaMemsetAsync(dev, 0, sizeof(Counts), st));
         auto pack = [&](int l) -> cudaError_t {
             const Atlas &a = atlas[l];
-            for (uint64_t z = 0; z < a.layers; z += a.per_buffer) {
-                const uint64_t nz = std::min(a.per_buffer, a.layers - z), per = (uint64_t)a.d * a.d;
-                const char *from = reinterpret_cast<const char *>(v->atlas[l]) + z * a.layer_bytes;
-                cudaError_t e = cudaMemcpy(base + need, from, nz * a.layer_bytes, cudaMemcpyHostToDevice);
+            if (!a.n) return cudaSuccess;
+            const uint64_t fit = (bytes - kFixed) / a.row;
+            for (uint64_t at = 0, step; at < a.rows; at += step) {
+                const uint64_t z = at / a.d, r = at % a.d, left = a.rows - at;
+                uint64_t layers = 1, rows = std::min({left, a.d - r, fit});  // block rows of a layer
+                if (r == 0 && rows == a.d) {
+                    layers = std::min(fit, left) / a.d;
+                    if (left > layers * a.d && (layers + 1) * a.d <= fit) layers++;  // the last one, partly filled
+                }
+                step = layers * rows;
+                const uint64_t first = at * a.d, count = std::min(step * a.d, a.n - first);
+                const size_t width = rows * a.texel_row >> a.log2;  // bytes of a texel layer of the piece
+                char *to = base + 256;
+                const char *from = reinterpret_cast<const char *>(v->atlas[l]) + (z << a.log2) * a.slice + r * (a.texel_row >> a.log2);
+                const size_t slices = layers << a.log2;
+                cudaError_t e = cudaSuccess;
+                if (width == a.slice) e = cudaMemcpy(to, from, slices * width, cudaMemcpyHostToDevice);
+                else if (a.slice <= INT32_MAX) e = cudaMemcpy2D(to, width, from, a.slice, width, slices, cudaMemcpyHostToDevice);
+                else  // beyond the largest pitch of a copy
+                    for (size_t k = 0; k < slices && e == cudaSuccess; k++)
+                        e = cudaMemcpy(to + k * width, from + k * a.slice, width, cudaMemcpyHostToDevice);
+                const wxk::ViewSlab s{reinterpret_cast<const uint32_t *>(to), v->dims[l][0], (uint32_t)(rows << a.log2), a.d, first, count};
+                to += step * a.texel_row;
+                const uint32_t *mask[2] = {nullptr, nullptr};
+                for (int m = 0; m < 2 && e == cudaSuccess; m++) {
+                    const uint32_t *src = m ? vals[l] : kids[l];
+                    if (!src) continue;
+                    to = base + (((size_t)(to - base) + 255) & ~(size_t)255);
+                    mask[m] = reinterpret_cast<const uint32_t *>(to);
+                    e = cudaMemcpy(to, src + first * a.words, count * a.words * 4, cudaMemcpyHostToDevice);
+                    to += count * a.words * 4;
+                }
                 if (e != cudaSuccess) return e;
-                const wxk::ViewSlab s{reinterpret_cast<const uint32_t *>(base + need), v->dims[l][0], v->dims[l][1], a.d,
-                                      z * per, std::min(nz * per, a.n - z * per)};
-                if (l < 2)
-                    e = wxk::pack_view_nodes(a.level, s, mask[2 * l], mask[2 * l + 1], (uint32_t)(l == 0 ? n4 : n3),
+                if (l < 2) {
+                    e = wxk::pack_view_nodes((int)a.log2, s, mask[0], mask[1], (uint32_t)(l == 0 ? n4 : n3),
                                              const_cast<uint32_t *>(l == 0 ? gr->g.slot5 : gr->g.slot4), &dev->flags, st);
-                else
-                    e = wxk::pack_view_leaves(s, mask[4], const_cast<uint8_t *>(gr->g.leaf), gr->ovf, gr->g.n_ovf,
-                                              &dev->n_ovf, st);
+                } else {
+                    e = wxk::sdf_count_clear(reinterpret_cast<const uint64_t *>(mask[1]), count * 8, &dev->clear, st);
+                    if (e == cudaSuccess)
+                        e = wxk::pack_view_leaves(s, mask[1], const_cast<uint8_t *>(gr->g.leaf), gr->ovf, gr->g.n_ovf,
+                                                  &dev->n_ovf, st);
+                }
                 if (e != cudaSuccess) return e;
             }
             return cudaSuccess;
         };
         for (int l = 0; l < 3; l++) WX_CUDA(ctx, pack(l));
-        WX_CUDA(ctx, wxk::sdf_count_clear(reinterpret_cast<const uint64_t *>(mask[4]), n3 * 8, &dev->clear, st));
         WX_CUDA(ctx, wxk::build_top_table(gr->g, st));
         WX_CUDA(ctx, cudaMemcpy(&h, dev, sizeof h, cudaMemcpyDeviceToHost));
         if (h.flags & 1u) return fail(ctx, WX_ERR_INVALID, "wx_grid_upload: child index in atlas out of range");

@@ -17,7 +17,7 @@ namespace {
 
 constexpr uint32_t kChild = 0x80000000u;
 
-// First texel of node idx in the slab of nodes that starts at `first` (a multiple of d * d).
+// First texel of node idx in the piece of nodes that starts at `first`: whole layers, or block rows of one.
 __device__ __forceinline__ size_t block_texel(const wxk::ViewSlab &s, uint64_t idx, uint32_t log2d) {
     const uint64_t r = idx - s.first, zb = r / ((uint64_t)s.d * s.d), q = r - zb * s.d * s.d, yb = q / s.d, xb = q - yb * s.d;
     return ((size_t)(zb << log2d) * s.h + (yb << log2d)) * s.w + (xb << log2d);
@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(256) k_pack_view_nodes(wxk::ViewSlab s, const 
     __syncthreads();
     uint32_t bad = 0;
     for (uint32_t o = threadIdx.x; o < N; o += 256u) {
-        const size_t w = (size_t)node * (N / 32) + (o >> 5);
+        const size_t w = (size_t)(node - s.first) * (N / 32) + (o >> 5);
         const uint32_t b = 1u << (o & 31u), v = buf[o ^ (o >> (2 * L))];
         uint32_t word = 0;
         if (!(vals[w] & b)) {
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(256) k_pack_view_leaves(wxk::ViewSlab s, const
 #pragma unroll 4
         for (uint32_t e = 0; e < 16; e++) {
             const uint32_t y = yb + (e & 1u) * 4u, z = e >> 1, o = (x << 6) | (y << 3) | z;
-            const bool val = (__ldg(vals + n * 16u + (o >> 5)) >> (o & 31u)) & 1u;
+            const bool val = (__ldg(vals + (n - s.first) * 16u + (o >> 5)) >> (o & 31u)) & 1u;
             const uint32_t v = val ? 0u : __ldg(t + ((size_t)z * s.h + y) * s.w);
             bytes[l * 512u + o] = (uint8_t)min(v, 255u);
             if (v >= 255u) {

@@ -137,14 +137,14 @@ cudaError_t sdf_levels(const SdfWork &w, uint32_t k0, uint32_t k1, int num_sms, 
 // Slot words and leaf bytes from the W sets of steps 0..kSdfWindow: after sdf_levels(1, kSdfWindow), before larger k.
 cudaError_t sdf_expand(const SdfWork &w, const uint32_t *cidx5, const uint32_t *cidx4, cudaStream_t st);
 
-// Packing of the flattened view (pack.cu): z slabs of an atlas in device memory, as block rows of nodes. The
-// texel of node idx's slot (x, y, z) is at ((idx' / d^2 * D + z) * h + (idx' / d % d * D + y)) * w + idx' % d * D + x
+// Packing of the flattened view (pack.cu): a piece of an atlas in device memory, whole layers of d * d nodes or some
+// block rows (d nodes) of one layer, with the masks of its nodes. The texel of node idx's slot (x, y, z) is at ((idx' / d^2 * D + z) * h + (idx' / d % d * D + y)) * w + idx' % d * D + x
 // with idx' = idx - first.
 struct ViewSlab {
     const uint32_t *texels;
-    uint32_t w, h;       // texture width and height
+    uint32_t w, h;       // width of the texture, height of the piece
     uint32_t d;          // nodes per row and rows per layer, as the shader derives them
-    uint64_t first, count;  // nodes of the slab
+    uint64_t first, count;  // nodes of the piece; first is a multiple of d
 };
 cudaError_t pack_view_nodes(int level, const ViewSlab &s, const uint32_t *kids, const uint32_t *vals, uint32_t nchild,
                             uint32_t *slot, uint32_t *flags, cudaStream_t st);
