@@ -30,6 +30,7 @@
 #include <thread>
 #include <vector>
 
+#include "launch_ring.h"
 #include "wx_alloc.h"
 #include "wx_common.h"
 #include "wx_kernels.h"
@@ -120,6 +121,8 @@ struct PixelOutputs {
     cudaStream_t stream;
     uintptr_t lo[2], hi[2];
 };
+std::mutex g_ring_mu;
+wxk::LaunchRing g_ring;
 constexpr size_t kPixelStreams = 256;  // records kept, oldest dropped first
 std::mutex g_pixel_mu;
 std::vector<PixelOutputs> g_pixel_outputs;
@@ -132,7 +135,9 @@ std::vector<PixelOutputs> g_pixel_outputs;
 // so no record can name its predecessor: frames on it always wait. NULL and
 // cudaStreamLegacy name the same stream.
 cudaError_t launch_pixel_tracked(const wxk::Job &job, const wxk::Tuning &t, int num_sms, PixelOutputs cur) {
-    if (cur.stream == cudaStreamPerThread) return wxk::launch_pixel(job, t, false, num_sms, cur.stream);
+    const uint64_t others = wxk::enter_launch(cur.device, cur.stream, job.tiles, (uint64_t)num_sms * wxk::kSplitWarps);
+    const uint32_t split = wxk::pixel_split(job.tiles, others, num_sms);
+    if (cur.stream == cudaStreamPerThread) return wxk::launch_pixel(job, t, false, split, cur.stream);
     if (cur.stream == cudaStreamLegacy) cur.stream = nullptr;
     auto meet = [](uintptr_t a0, uintptr_t a1, uintptr_t b0, uintptr_t b1) {
         return a0 < a1 && b0 < b1 && a0 < b1 && b0 < a1;
@@ -151,7 +156,7 @@ cudaError_t launch_pixel_tracked(const wxk::Job &job, const wxk::Tuning &t, int 
     } else if (v.size() >= kPixelStreams) {
         v.erase(v.begin());
     }
-    const cudaError_t e = wxk::launch_pixel(job, t, disjoint, num_sms, cur.stream);
+    const cudaError_t e = wxk::launch_pixel(job, t, disjoint, split, cur.stream);
     if (e == cudaSuccess) v.push_back(cur);  // after a failed launch the stream's last kernel is unknown
     return e;
 }
@@ -400,6 +405,14 @@ wxk::Job make_job(const wx_grid *grid, const wx_state_uniform &s, uint32_t width
 }
 
 }  // namespace
+
+uint64_t wxk::enter_launch(int device, cudaStream_t st, uint64_t tiles, uint64_t enough) {
+    static thread_local char thread;
+    if (st == cudaStreamLegacy) st = nullptr;
+    std::lock_guard<std::mutex> lock(g_ring_mu);
+    return g_ring.enter(device, reinterpret_cast<uintptr_t>(st),
+                        st == cudaStreamPerThread ? reinterpret_cast<uintptr_t>(&thread) : 0, tiles, enough);
+}
 
 void wxk::ctx_device_info(const wx_ctx *ctx, int *device, int *num_sms) {
     *device = ctx->device;
@@ -1065,6 +1078,7 @@ int wx_render(wx_ctx *ctx, const wx_grid *grid, const wx_state_uniform *state, u
             const cudaError_t e = launch_pixel_tracked(job, ctx->tuning, ctx->num_sms, cur);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "wxk::launch_pixel");
         } else {
+            wxk::enter_launch(ctx->device, st, job.tiles);
             WX_CUDA(ctx, wxk::launch_persistent(job, ctx->take_counter(), ctx->tuning, ctx->num_sms, st));
         }
         // Copy back only the dispatched region; the rest of a host buffer is untouched.
@@ -1140,6 +1154,7 @@ int wx_render_batch(wx_ctx *ctx, const wx_frame *frames, uint32_t n, void *strea
         WX_CUDA(ctx, cudaMemcpyAsync(ctx->jobs_dev, ctx->jobs_host, jobs.size() * sizeof(wxk::Job),
                                      cudaMemcpyHostToDevice, st));
         WX_CUDA(ctx, cudaEventRecord(ctx->jobs_done, st));
+        wxk::enter_launch(ctx->device, st, total);
         WX_CUDA(ctx, wxk::launch_batched(ctx->jobs_dev, (uint32_t)jobs.size(), tab, total, ctx->take_counter(), ctx->tuning,
                                          ctx->num_sms, wxk::all_modes(jobs.data(), jobs.size()), st));
         return WX_OK;
@@ -1197,6 +1212,7 @@ int wx_batch_launch(wx_batch *b, void *stream) {
     return wx::guard("wx_batch_launch", [&]() -> int {
         if (!b) return WX_ERR_INVALID;
         WX_CUDA(b->ctx, cudaSetDevice(b->ctx->device));
+        wxk::enter_launch(b->ctx->device, static_cast<cudaStream_t>(stream), b->total_tiles);
         WX_CUDA(b->ctx, cudaGraphLaunch(b->exec, static_cast<cudaStream_t>(stream)));
         return WX_OK;
     });

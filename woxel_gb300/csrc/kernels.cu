@@ -161,7 +161,7 @@ __device__ __forceinline__ void render_pixel(const Job &J, const DevGrid &G, uin
 //
 // split: 2^split warps share a tile, each with the first 32 >> split of its lanes. A small frame leaves the chip idle
 // and takes as long as its slowest warp; with fewer rays a warp, an iteration resolves fewer levels in turn and no ray
-// waits for 31 others. See pixel_split.
+// waits for 31 others. See pixel_split (launch_ring.h).
 template <int kModes>
 __global__ void WX_PIXEL_BOUNDS k_pixel(const __grid_constant__ Job job, uint32_t ntiles, uint32_t disjoint, uint32_t split) {
     if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -504,17 +504,8 @@ int max_blocks_per_sm(int kernel, bool batched, int warps_per_block) {
     return batched ? blocks_for(k_persistent<kTableGrid, kBase>, threads) : blocks_for(k_persistent<kOneJob, kBase>, threads);
 }
 
-// Warps a tile: as many, up to 8, as keep the frame's warps within 28 an SM (of 64). Mode 3 over 500 spheres and over
-// one, queued frames, us at 1, 2, 4 and 8 warps a tile: 192 tiles 94, 63, 56, 51 and 44, 30, 27, 25; 600 tiles 74, 65,
-// 62, 62 and 34, 30, 27, 28; 2048 tiles 82, 74, 77, 101 and 33, 32, 37, 60; 3750 tiles 85, 84, 96, 152 and 34, 36, 53, 99.
-static uint32_t pixel_split(uint32_t tiles, int num_sms) {
-    uint32_t s = 0;
-    while (s < 3u && ((uint64_t)tiles << (s + 1u)) <= (uint64_t)num_sms * 28u) s++;
-    return s;
-}
-
-cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, int num_sms, cudaStream_t st) {
-    const uint32_t wpb = (uint32_t)t.warps_per_block, split = pixel_split(job.tiles, num_sms);
+cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, uint32_t split, cudaStream_t st) {
+    const uint32_t wpb = (uint32_t)t.warps_per_block;
     // Programmatic dependent launch: back-to-back frames on one stream overlap
     // the previous frame's last blocks with this frame's march (the kernel's
     // stores wait for the previous kernel; see render_pixel).
@@ -781,6 +772,7 @@ int noalloc_render(int device, const wx_frame *frames, uint32_t n, cudaStream_t 
     uint32_t *counter = reinterpret_cast<uint32_t *>(d->scratch);
     wxk::Tuning t;  // defaults; launch_batched clears the counter (it keeps the last call's value otherwise)
     const cudaError_t e = wxk::launch_batched(jobs_dev, njobs, tab, (uint32_t)tiles, counter, t, d->num_sms, all, st);
+    wxk::enter_launch(device, st, tiles);
     if (e != cudaSuccess) return noalloc_fail(WX_ERR_CUDA, "wx_render_batch_noalloc: launch failed");
     return WX_OK;
 }

@@ -248,6 +248,7 @@ struct wx_server {
         wxk::Tuning t;
         cudaError_t e = cudaMemcpyAsync(s.jobs_dev, s.jobs_host, n * sizeof(wxk::Job), cudaMemcpyHostToDevice, s.stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(s.counter, 0, 2 * sizeof(uint32_t), s.stream);
+        wxk::enter_launch(device, s.stream, tiles);
         if (e == cudaSuccess)
             e = wxk::launch_batched(s.jobs_dev, n, tab, tiles, s.counter, t, num_sms, wxk::all_modes(s.jobs_host, n),
                                     s.stream, cancel_dev, s.counter + 1);

@@ -69,8 +69,8 @@ cudaError_t init_device_tables();
 cudaError_t build_top_table(const DevGrid &g, cudaStream_t st);
 int max_blocks_per_sm(int kernel, bool batched, int warps_per_block);
 // disjoint: the job's outputs do not overlap those of the previous kernel on st,
-// a k_pixel launch (see k_pixel); false is always safe.
-cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, int num_sms, cudaStream_t st);
+// a k_pixel launch (see k_pixel); false is always safe. split: 2^split warps share a tile (not in k_wave).
+cudaError_t launch_pixel(const Job &job, const Tuning &t, bool disjoint, uint32_t split, cudaStream_t st);
 cudaError_t launch_persistent(const Job &job, uint32_t *ctr, const Tuning &t, int num_sms, cudaStream_t st);
 // all: some job renders mode 4 or 5 (the kernels compiled for every mode).
 // cancel (may be NULL): the table the jobs' cancel_slot index; skipped (may be
@@ -79,6 +79,9 @@ cudaError_t launch_persistent(const Job &job, uint32_t *ctr, const Tuning &t, in
 cudaError_t launch_batched(const Job *jobs_dev, uint32_t njobs, const GridTable &tab, uint32_t total_tiles, uint32_t *ctr,
                            const Tuning &t, int num_sms, bool all, cudaStream_t st,
                            const uint32_t *cancel = nullptr, uint32_t *skipped = nullptr);
+// Enters a launch of `tiles` into the process's ring of launches (launch_ring.h); returns the tiles of the other streams of its
+// device, or a number above `enough`.
+uint64_t enter_launch(int device, cudaStream_t st, uint64_t tiles, uint64_t enough = 0);
 // Enters the job's grid into the table (unless it has overflowed: n = kTableGrids + 1) and its place into job.order.
 void index_grid(Job &job, GridTable &tab);
 // Modes 4 (glossy) and 5 (zero crossing) need the kernels compiled for every mode.
