@@ -323,7 +323,8 @@ __device__ __forceinline__ uint32_t node_step(const SdfWork &S, uint32_t k, uint
     using G = Geo<L>;
     const SdfLevel &V = S.lv[5 - L];
     const uint32_t c = task / (G::kNode / 32), r = (task % (G::kNode / 32)) * 32u + lane;
-    if (k > wxk::kSdfWindow + 1u && V.act[c] + 1u < k) return 0;
+    // Other CTAs set act while it is read: the vote makes the lanes agree, as the votes below need.
+    if (k > wxk::kSdfWindow + 1u && !__any_sync(~0u, V.act[c] + 1u >= k)) return 0;
     const Step st = step_of(V, k);
     const int x = (int)(r / G::kSlice), yq = (int)(r % G::kSlice);
     uint32_t n[9];
