@@ -19,6 +19,12 @@ namespace {
 struct Mem {
     template <class T>
     T add(T *p, T v) const { return __atomic_fetch_add(p, v, __ATOMIC_RELAXED); }
+    uint32_t count(uint32_t *p, uint32_t n) const {
+        uint32_t v = load(p);
+        while (!__atomic_compare_exchange_n(p, &v, v + 1u < n ? v + 1u : 0u, true, __ATOMIC_RELAXED, __ATOMIC_RELAXED)) {
+        }
+        return v;
+    }
     template <class T>
     T load(const T *p) const { return __atomic_load_n(p, __ATOMIC_RELAXED); }
     void store(uint32_t *p, uint32_t v) const { __atomic_store_n(p, v, __ATOMIC_RELAXED); }

@@ -358,8 +358,13 @@ __device__ __forceinline__ uint32_t node_step(const SdfWork &S, uint32_t k, uint
 struct StepsMem {
     template <class T>
     __device__ __forceinline__ T add(T *p, T v) const { return atomicAdd(p, v); }
+    __device__ __forceinline__ uint32_t count(uint32_t *p, uint32_t n) const { return atomicInc(p, n - 1u); }
     __device__ __forceinline__ uint32_t load(const uint32_t *p) const { return ld_relaxed(p); }
-    __device__ __forceinline__ unsigned long long load(unsigned long long *p) const { return atomicAdd(p, 0ull); }
+    __device__ __forceinline__ unsigned long long load(const unsigned long long *p) const {
+        unsigned long long v;
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+        return v;
+    }
     __device__ __forceinline__ void store(uint32_t *p, uint32_t v) const { atomicExch(p, v); }
     __device__ __forceinline__ void fence() const { __threadfence(); }
     // Polls are relaxed: an acquire would empty the SM's L1 under the CTAs still at work (the fence after them acquires).

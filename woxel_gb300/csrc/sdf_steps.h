@@ -9,8 +9,9 @@
 // (the levels that still have cells) is part of the same word: no CTA derives it from counters that
 // others are changing.
 //
-// M: relaxed loads and stores, an atomic add that returns the old value, a fence that orders all
-// earlier accesses of the CTA before all later ones, and a pause. The kernel's are in sdf.cu.
+// M: relaxed loads and stores, an atomic add that returns the old value, an atomic count from 0 to
+// n - 1 and round again that does too, a fence that orders all earlier accesses of the CTA before all
+// later ones, and a pause. The kernel's are in sdf.cu.
 #pragma once
 
 #include <cstdint>
@@ -51,10 +52,11 @@ constexpr uint32_t kStepsStartPolls = 32u;
 
 template <class M>
 WX_STEPS uint32_t steps_publish(M m, SdfCtl *c, uint32_t k) {
-    uint32_t done = 0;
-    for (uint32_t l = 0; l < 3u; l++) done |= m.load(&c->left[l]) == 0ull ? 1u << l : 0u;
-    const uint32_t w = steps_word(k, m.load(&c->started), m.load(&c->error) ? kStepsAllDone : done);
-    m.fence();
+    // All loads in flight together: every other CTA waits for this one.
+    const uint32_t ctas = m.load(&c->started), error = m.load(&c->error);
+    const unsigned long long n5 = m.load(&c->left[0]), n4 = m.load(&c->left[1]), n3 = m.load(&c->left[2]);
+    const uint32_t done = (n5 ? 0u : 1u) | (n4 ? 0u : 2u) | (n3 ? 0u : 4u);
+    const uint32_t w = steps_word(k, ctas, error ? kStepsAllDone : done);
     m.store(&c->release, w);
     return w;
 }
@@ -92,11 +94,10 @@ template <class M>
 WX_STEPS uint32_t steps_next(M m, SdfCtl *c, uint32_t ticket, uint32_t w, uint32_t k1, uint32_t limit) {
     const uint32_t k = steps_k(w) + 1u;
     m.fence();
-    if (m.add(&c->arrived, 1u) != steps_ctas(w) - 1u) return steps_wait(m, c, ticket, k, k1, limit);
-    m.fence();
+    if (m.count(&c->arrived, steps_ctas(w)) != steps_ctas(w) - 1u) return steps_wait(m, c, ticket, k, k1, limit);
+    m.fence();  // before the release: the count is back at 0, and the other CTAs' writes are before this one's release
     for (uint32_t l = 0; l < 3u; l++)
         if (!((steps_done(w) >> l) & 1u)) c->last[l] = k;
-    m.store(&c->arrived, 0u);
     return steps_publish(m, c, k);
 }
 
