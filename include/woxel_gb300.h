@@ -102,7 +102,7 @@ typedef struct wx_vdb345_view {
 
 typedef struct wx_grid_info {
     uint64_t n5, n4, n3;           /* node counts per level */
-    uint64_t device_bytes;         /* bytes of device node pools */
+    uint64_t device_bytes;         /* bytes of device node pools, the 1 MB top table included */
     uint64_t active_voxels;        /* popcount of the leaf value masks */
 } wx_grid_info;
 

@@ -331,7 +331,7 @@ class Context:
         check(lib().wx_ctx_set_tuning(self._h, C.byref(t)), self._h)
 
     def set_sdf_wait_limit(self, polls: int) -> None:
-        """Bound of the GPU SDF build's dependency waits (polls 256 ns apart; 0 = default, about 2 s)."""
+        """Bound of the GPU SDF build's waits between steps (polls 256 ns apart; 0 = default, about 2 s)."""
         check(lib().wx_ctx_set_sdf_wait_limit(self._h, polls), self._h)
 
     def autotune(self, frames: Sequence, candidates: Optional[Sequence[dict]] = None, reps: int = 3) -> dict:

@@ -6,11 +6,14 @@
 //          n5 x int4         N5 origins (root keys) in DFS order
 //          dim.x*dim.y*dim.z u32  dense root-key table over the box of N5 keys
 //                            (origin >> 12) starting at lo: N5 index + 1, 0 = none
+//   top    64^3 u32          the slot5 words of the box [-4096, 4096)^3 by position, 32 where there is no N5: just
+//                            before slot5, where the kernels address it (slot5 - kTopWords)
 //   slot5  n5 x 32768 u32    per N4-sized slot: child flag|N4 index, or skip distance
 //   slot4  n4 x  4096 u32    per N3-sized slot: child flag|N3 index, or skip distance
 //   leaf   n3 x   512 u8     per voxel: 0 for an active voxel (a hit), else the skip
 //                            distance, 255 meaning "at least 255: look it up in ovf"
-//   ovf    n_ovf x (u32,u32) (voxel key = leaf << 9 | offset, exact distance), sorted
+//   ovf    n_ovf x (u32,u32) (voxel key = leaf << 9 | offset, exact distance), sorted; in a block of its
+//                            own where the build learns n_ovf after the pools (GPU build, upload)
 // A slot word folds the reference's three reads per level (child-mask word,
 // value-mask word, atlas texel; raycast.comp.wgsl:422-429, :453-461,
 // :483-489) into one load that decides hit / descend / skip. Leaf distances

@@ -178,9 +178,11 @@ __global__ void WX_PIXEL_BOUNDS k_pixel(const __grid_constant__ Job job, uint32_
 // warp are idle, so the march runs with most lanes busy; the ray's result goes
 // to the warp's shared-memory slots and the unit's pixels are shaded 32 at a
 // time once every ray has ended. The unit's shadow rays (mode 3) are queued in
-// the same slots and marched the same way. Every ray performs exactly the
-// ray_step sequence it performs in k_pixel, so pixels and hit records are
-// identical. Launched like k_pixel (programmatic dependent launch).
+// the same slots and marched the same way. Its rays advance by ray_step, an
+// iteration at a time, where k_pixel runs march_loop to the ray's end; both perform
+// the shader's iterations bit for bit, so pixels and hit records are identical.
+// 8 frames of 1000 spheres at 1080p in mode 3: 5.7 ms at 2 rays a lane, 2.6 in
+// k_pixel. Launched like k_pixel (programmatic dependent launch).
 // ---------------------------------------------------------------------------
 constexpr uint32_t kWaveWords = 5;               // slot: p.xyz, info, node | queued shadow ray: src.xyz, pixel, colour
 constexpr uint32_t kSlotInvalid = 0xFFFFFFFFu;   // info of a pixel outside the dispatched region

@@ -564,7 +564,8 @@ __device__ __forceinline__ void march_loop(const DevGrid &g, Loop &s, F3 dir, fl
 // kOct: a loop for each of the eight sign patterns of a direction, in which step01 and the nudge are constants (8 frames
 // of 2000 spheres 3.11 -> 3.04 ms, 2 noise frames 2.09 -> 2.04 ms; a tile's rays rarely differ). The persistent kernels
 // have rays of several frames on an SM at a time, and nine loops are too much code for them (12.5 -> 12.9 ms); so they
-// are beside the zero-crossing search (0.525 -> 0.56 ms).
+// are beside the zero-crossing search (0.525 -> 0.56 ms). The glossy chain's shadow rays have them in every kernel: 24
+// frames of all six modes in one batch 4.21 -> 4.07 ms, of modes 3 and 4 5.00 either way, of modes 3 and 5 5.09 -> 5.23 ms.
 // oct says which direction components are negative (bits x, y, z) for every lane that calls together, or is 8 where they differ.
 template <bool kOct>
 __device__ __forceinline__ March hdda(const DevGrid &g, F3 src, F3 dir, uint32_t oct = 8u) {

@@ -47,8 +47,8 @@ struct Job {
     uint32_t cancel_slot, cancel_id;
 };
 
-// The distinct grids of a batched launch, a kernel parameter; n = 0 when there are more than kTableGrids (the jobs'
-// own copies are then used).
+// The distinct grids of a batched launch, a kernel parameter; n = kTableGrids + 1 when there are more than kTableGrids
+// (the jobs' own copies are then used).
 constexpr uint32_t kTableGrids = 64;
 struct GridTable {
     DevGrid g[kTableGrids];
