@@ -34,7 +34,7 @@
 // when it or one of its 26 neighbours changed in the step before (act = the last
 // such step), and store a cell's distance when it enters W. The barrier's wait is
 // bounded; on the bound an error flag ends the kernel.
-// 2000-sphere grid (476,014 leaves, 14 steps, the leaves done after 7): 0.90 ms, where the sweeps
+// 2000-sphere grid (476,014 leaves, 14 steps, the leaves done after 7): 0.88 ms with k_expand_*, where the sweeps
 // in the sweep's order (one CTA a container, a ready queue, 50 barriers a leaf) took 27.4 ms, bound
 // by the chain of containers that wait for one another.
 // Distances are small: a cell at distance k lies in a solid cube of containers
@@ -374,7 +374,7 @@ struct StepsMem {
 // Steps k0 to k1, or fewer when every cell has its distance. A level takes no part once none is left in it. The CTAs
 // that run share each step among them (sdf_steps.h).
 constexpr uint32_t kLeafChunk = 8;  // groups of three leaves a warp takes at a time, looked over with one load
-// Bound by the latency of its gathers. 2000-sphere grid, 14 steps: 0.76 ms with the two k_expand_* another 0.14 ms; as
+// Bound by the latency of its gathers. 2000-sphere grid, 14 steps: 0.77 ms, and k_expand_* another 0.11 ms; as
 // one kernel that stored every distance by an atomic and marked the neighbours of every change from the first step on,
 // 2.1 ms (of a full step's 670 us the marks took 330 and the atomics 190). 6 CTAs an SM at 40 registers: 1.96 ms for
 // the whole build; 2.04 at 4 CTAs (64 registers), 2.14 at 5, 2.47 at 8 (spills).

@@ -329,8 +329,10 @@ int wx_server_create(wx_ctx *ctx, const wx_server_config *cfg, wx_server **out) 
         wx_server_config c = *cfg;
         if (c.max_inflight == 0) c.max_inflight = 2;
         // Default slice: four 1080p frames. Measured at saturation (5000 req/s over the 8
-        // benchmark grids): 3.58 Grays/s at 16,384 tiles per launch, 5.62 at 65,536, 5.90 at
-        // 262,144 and 5.94 at 1,048,576, with p50/p99 at 200-2000 req/s unchanged or better.
+        // benchmark grids): 4.52 Grays/s at 16,384 tiles per launch, 7.79 at 65,536, 8.35 at
+        // 262,144 and 8.36 at 1,048,576; at 1000 and 2000 req/s p50/p99 are the same from 65,536 on
+        // (0.45 / 2.8 ms and 0.8-0.9 / 4.7-5.0 ms). Launches in flight: 7.12 with one, 8.35 with
+        // two, 8.42 with three or four.
         if (c.slice_tiles == 0) c.slice_tiles = 262144;
         if (c.max_frames == 0) c.max_frames = 256;
         if (c.max_inflight > 8 || c.max_frames > 1024)
