@@ -156,8 +156,9 @@ const char *wx_last_error(const wx_ctx *ctx);
 /* ---- grids: replace the atlas/mask upload (wgpu_context.rs:101-159, 506-573) ---- */
 /* Drop-in: repack the Rust side's flattened view into device node pools. The
  * atlases and masks are copied and packed in pieces: temporary device memory is
- * at most 256 MB, less for a small view or where the device has less beside the
- * grid, down to one row of nodes of an atlas. */
+ * at most 64 MB (or one row of nodes of an atlas, if that is more), less for a
+ * small view or where the device has less beside the grid; the context keeps at
+ * most 32 MB of it from the next synchronisation on, until it is destroyed. */
 int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *view, wx_grid **out);
 /* Native: compute the per-level SDF (vdb345.rs:290-670) on the host and pack
  * the pools directly from a topology, without the padded atlas. */

@@ -39,6 +39,12 @@
 #include "wx_kernels.h"
 
 namespace {
+// Temporary buffer of wx_grid_upload, at most. 200 spheres (104 MB of leaf texels) and the first frame: 1.34 ms at 256 and at 64 MB,
+// 1.44 at 32; on a new state 2.1, 2.0 and 2.0 ms; 1000 spheres (520 MB) 3.8, 3.9, 4.1 ms and 4.6 at 16.
+constexpr size_t kUploadBuffer = (size_t)64 << 20;
+// What the context's pool keeps of it at a synchronisation. Pools map 32 MB at a time: with nothing kept, an upload after a
+// synchronisation takes 0.49 ms for two voxels, 0.62 ms for 40 spheres and 1.27 ms for 200, so 0.34, 0.48 and 1.18 ms.
+constexpr size_t kUploadKeep = (size_t)32 << 20;
 constexpr uint32_t kCounterSlots = 1u << 16;  // one work counter per in-flight launch (ring)
 }
 
@@ -50,12 +56,15 @@ struct wx_ctx {
     uint32_t *counters = nullptr;       // kCounterSlots device counters
     uint32_t next_counter = 0;
     unsigned long long *check = nullptr;  // division self-check results
+    cudaMemPool_t pool = nullptr;       // for wx_grid_upload's buffer; keeps at most kUploadKeep
     void *stage = nullptr;              // device staging for host-memory outputs
     size_t stage_bytes = 0;
     wxk::Job *jobs_dev = nullptr;       // job table of the one-shot batch entry point
     size_t jobs_cap = 0;
     wxk::Job *jobs_host = nullptr;      // pinned staging for that table
     cudaEvent_t jobs_done = nullptr;    // last one-shot batch's table copy
+    std::vector<uint32_t> top;          // the top table of the last host build (upload_pools)
+    uint32_t top_octants = 0;           // its octants that are not 32 throughout
     uint32_t sdf_spins = wxk::kSdfSpinLimit;  // bound of the waits in the GPU SDF's step control
     uint32_t *take_counter() {
         uint32_t *c = counters + next_counter;
@@ -185,20 +194,31 @@ void *pinned_device_alias(void *p) {
     return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
-// A device allocation freed on scope exit (temporaries of wx_grid_build_gpu and wx_grid_upload).
+// A device allocation freed on scope exit (temporaries of wx_grid_build_gpu).
 struct DevBuf {
     void *p = nullptr;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    ~DevBuf() { release(); }
-    void release() {
+    ~DevBuf() {
         if (p) cudaFree(p);
-        p = nullptr;
     }
     template <class T>
     T *as() const {
         return static_cast<T *>(p);
+    }
+};
+// The same from a memory pool, in the order of the legacy stream (the temporary of wx_grid_upload): nothing waits for other
+// streams.
+struct StreamBuf {
+    void *p = nullptr;
+    StreamBuf() = default;
+    StreamBuf(const StreamBuf &) = delete;
+    StreamBuf &operator=(const StreamBuf &) = delete;
+    ~StreamBuf() { release(); }
+    void release() {
+        if (p) cudaFreeAsync(p, nullptr);
+        p = nullptr;
     }
 };
 
@@ -347,6 +367,7 @@ int upload_pools(wx_ctx *ctx, const std::vector<int4> &o5, const uint32_t *s5, c
     std::vector<uint8_t> leaf;
     std::vector<uint2> ovf;
     try {
+        if (ctx->top.empty()) ctx->top.assign(wxk::kTopWords, 32u);
         leaf.resize(n3 * wx::kN3Slots);
         const unsigned np = n3 < 4096 ? 1u : std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
         std::vector<std::vector<uint2>> parts(np);
@@ -375,8 +396,21 @@ int upload_pools(wx_ctx *ctx, const std::vector<int4> &o5, const uint32_t *s5, c
     if (e == cudaSuccess && n3) e = cudaMemcpy((void *)gr->g.leaf, leaf.data(), leaf.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !ovf.empty())
         e = cudaMemcpy((void *)gr->g.ovf, ovf.data(), ovf.size() * 8, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = wxk::build_top_table(gr->g, nullptr);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    // The top table is made here, not by build_top_table: no kernel to wait for behind renders on other streams.
+    for (uint32_t oct = 0; oct < 8u; oct++) {
+        const uint32_t ox = oct >> 2, oy = (oct >> 1) & 1u, oz = oct & 1u;
+        uint64_t i = 0;  // the first N5 there, as root_find gives it
+        while (i < n5 && !(o5[i].x == (int)ox * 4096 - 4096 && o5[i].y == (int)oy * 4096 - 4096 && o5[i].z == (int)oz * 4096 - 4096)) i++;
+        if (i == n5 && !((ctx->top_octants >> oct) & 1u)) continue;
+        ctx->top_octants = (ctx->top_octants & ~(1u << oct)) | (i < n5 ? 1u << oct : 0u);
+        for (uint32_t xy = 0; xy < 1024u; xy++) {
+            uint32_t *row = &ctx->top[((ox * 32u + (xy >> 5)) << 12) | ((oy * 32u + (xy & 31u)) << 6) | (oz * 32u)];
+            if (i < n5) memcpy(row, s5 + i * wx::kN5Slots + xy * 32u, 32 * sizeof(uint32_t));
+            else std::fill(row, row + 32, 32u);
+        }
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpy((void *)(gr->g.slot5 - wxk::kTopWords), ctx->top.data(), ctx->top.size() * 4, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         free_grid(gr);
         return cuda_fail(ctx, e, "cudaMemcpy(node pools)");
@@ -484,6 +518,7 @@ int wx_ctx_destroy(wx_ctx *ctx) {
             cudaEventSynchronize(ctx->jobs_done);
             cudaEventDestroy(ctx->jobs_done);
         }
+        if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
         if (ctx->stage) cudaFree(ctx->stage);
         if (ctx->counters) cudaFree(ctx->counters);
         if (ctx->check) cudaFree(ctx->check);
@@ -871,7 +906,7 @@ int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *v, wx_grid **out) {
             o5[i] = make_int4(o[0], o[1], o[2], 0);
         }
         // Piece by piece, an atlas and its nodes' masks are copied to the device and packed there (pack.cu). A piece is whole
-        // layers of d * d nodes, or block rows (d nodes) of one layer: as many as fit the buffer, 256 MB where the
+        // layers of d * d nodes, or block rows (d nodes) of one layer: as many as fit the buffer, 64 MB where the
         // device has that beside the grid, less where it has not, down to one block row.
         const uint32_t *const kids[3] = {v->kids5, v->kids4, nullptr}, *const vals[3] = {v->vals5, v->vals4, v->vals3};
         struct Atlas {
@@ -891,15 +926,25 @@ int wx_grid_upload(wx_ctx *ctx, const wx_vdb345_view *v, wx_grid **out) {
             least = std::max(least, kFixed + a.row);
             most = std::max(most, kFixed + a.row * (a.rows < a.d ? a.rows : (a.rows + a.d - 1) / a.d * a.d));
         }
+        if (!ctx->pool) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location = {cudaMemLocationTypeDevice, ctx->device};
+            WX_CUDA(ctx, cudaMemPoolCreate(&ctx->pool, &props));
+            uint64_t keep = kUploadKeep;
+            WX_CUDA(ctx, cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        }
         wx_grid *gr = nullptr;
-        DevBuf tmp;
-        size_t bytes = std::max(least, std::min(most, (size_t)256 << 20));
+        StreamBuf tmp;
+        size_t bytes = std::max(least, std::min(most, kUploadBuffer));
         for (;; bytes = std::max(least, bytes / 2)) {
-            const cudaError_t e = wx::dev_alloc(&tmp.p, bytes);
+            const cudaError_t e = wx::dev_alloc_async(&tmp.p, bytes, ctx->pool, nullptr);
             rc = e == cudaSuccess ? alloc_grid(ctx, o5, n5, n4, n3, 0, &gr) : cuda_fail(ctx, e, "cudaMalloc(upload buffer)");
             if (rc == WX_OK) break;
             tmp.release();
             if (rc != WX_ERR_OOM || bytes == least) return rc;
+            cudaStreamSynchronize(nullptr);
+            cudaMemPoolTrimTo(ctx->pool, 0);
             cudaGetLastError();
         }
         GridGuard guard{gr};
